@@ -1,24 +1,14 @@
-// Shared-memory batched complex FFT used by the horizontal transform kernels.
-//
-// Layout: one CTA transforms B independent length-N sequences held in shared
-// memory as data[n * B + b] (batch innermost).  B is chosen so a row of B
-// complex values is 128 bytes (8 double2 or 16 float2): consecutive threads
-// then touch consecutive 8/16-byte words, which makes every pass free of bank
-// conflicts and lets the global loads and stores that fill and drain the
-// buffer move whole 32-byte sectors when the batch index is the innermost
-// global index too (planes are innermost in the WVM layout).
+// Complex arithmetic, small DFTs and the warp-level FFTs of the kernels.
 //
 // Algorithm: Stockham auto-sort, decimation in time.  Pass p with current
 // sub-transform size Ns and radix R: butterfly j reads x[j + r*N/R], multiplies
 // by the twiddle w^(r*(j mod Ns)) with w = exp(sign*2*pi*i/(Ns*R)), applies a
 // length-R DFT and writes x[(j/Ns)*Ns*R + (j mod Ns) + r*Ns].  Output is in
-// natural order.  Every thread owns exactly eight elements per pass (one
-// radix-8 butterfly, two radix-4 or four radix-2 butterflies), so a pass reads
-// all its inputs into registers, synchronises, and writes in place.
+// natural order.
 //
 // Twiddles come from a table tw[k] = exp(-2*pi*i*k/N), k in [0, N), generated on
-// the host in long double and rounded to T (see twiddles.cpp); the inverse
-// direction uses their conjugates.
+// the host in long double and rounded to T; the inverse direction uses their
+// conjugates.
 
 #pragma once
 
@@ -121,125 +111,6 @@ template <int SIGN, typename V>
 __device__ __forceinline__ V twiddle(const V* __restrict__ tw, int k) {
     const V w = __ldg(tw + k);
     return SIGN < 0 ? w : cconj(w);
-}
-
-constexpr int fft_threads(int N) { return N >= 8 ? N / 8 : 1; }
-
-// Transform B sequences of length N in shared memory, element (n, b) at
-// data[n * LD + b] (LD = B, or B + 1 where callers also walk along n).  Must
-// be called by all fft_threads(N)*B threads (tid in [0, that)); other threads
-// of the CTA must still reach the __syncthreads() calls, which is why
-// `active` exists.
-template <typename T, int N, int B, int SIGN, int LD = B>
-__device__ __forceinline__ void fft_smem(cx<T>* data, const cx<T>* __restrict__ tw, int tid, bool active) {
-    using V = cx<T>;
-    if constexpr (N == 1) {
-        return;
-    } else if constexpr (N < 8) {
-        // Tiny lengths (rows of an 8-point grid): one thread per sequence.
-        if (active) {
-            V v[N];
-            const int b = tid;
-#pragma unroll
-            for (int n = 0; n < N; ++n) v[n] = data[n * LD + b];
-            if constexpr (N == 2) {
-                dft2<SIGN>(v[0], v[1]);
-            } else {
-                V t0 = v[0], t1 = v[1], t2 = v[2], t3 = v[3];
-                dft4<SIGN>(t0, t1, t2, t3);
-                v[0] = t0;
-                v[1] = t1;
-                v[2] = t2;
-                v[3] = t3;
-            }
-#pragma unroll
-            for (int n = 0; n < N; ++n) data[n * LD + b] = v[n];
-        }
-        __syncthreads();
-    } else {
-        const int b = tid % B;
-        const int j = tid / B;  // butterfly group in [0, N/8)
-        int Ns = 1;
-#pragma unroll
-        for (int pass = 0; pass < 12; ++pass) {
-            if (Ns * 8 > N) break;
-            V v[8];
-            if (active) {
-#pragma unroll
-                for (int r = 0; r < 8; ++r) v[r] = data[(j + r * (N / 8)) * LD + b];
-                const int k = j % Ns;
-                if (Ns > 1) {
-                    const int step = k * (N / (Ns * 8));
-#pragma unroll
-                    for (int r = 1; r < 8; ++r) v[r] = cmul(v[r], twiddle<SIGN>(tw, step * r));
-                }
-                dft8<SIGN>(v);
-            }
-            __syncthreads();
-            if (active) {
-                const int k = j % Ns;
-                const int base = (j / Ns) * Ns * 8 + k;
-#pragma unroll
-                for (int r = 0; r < 8; ++r) data[(base + r * Ns) * LD + b] = v[r];
-            }
-            __syncthreads();
-            Ns *= 8;
-        }
-        constexpr int rest = [] {
-            int ns = 1;
-            while (ns * 8 <= N) ns *= 8;
-            return N / ns;
-        }();
-        if constexpr (rest == 4) {
-            // Final radix-4 pass: Ns = N/4, two butterflies per thread.
-            constexpr int ns = N / 4;
-            V v[8];
-            if (active) {
-#pragma unroll
-                for (int s = 0; s < 2; ++s) {
-                    const int jj = j + s * (N / 8);
-#pragma unroll
-                    for (int r = 0; r < 4; ++r) v[4 * s + r] = data[(jj + r * ns) * LD + b];
-#pragma unroll
-                    for (int r = 1; r < 4; ++r) v[4 * s + r] = cmul(v[4 * s + r], twiddle<SIGN>(tw, jj * r));
-                    dft4<SIGN>(v[4 * s], v[4 * s + 1], v[4 * s + 2], v[4 * s + 3]);
-                }
-            }
-            __syncthreads();
-            if (active) {
-#pragma unroll
-                for (int s = 0; s < 2; ++s) {
-                    const int jj = j + s * (N / 8);
-#pragma unroll
-                    for (int r = 0; r < 4; ++r) data[(jj + r * ns) * LD + b] = v[4 * s + r];
-                }
-            }
-            __syncthreads();
-        } else if constexpr (rest == 2) {
-            // Final radix-2 pass: Ns = N/2, four butterflies per thread.
-            constexpr int ns = N / 2;
-            V v[8];
-            if (active) {
-#pragma unroll
-                for (int s = 0; s < 4; ++s) {
-                    const int jj = j + s * (N / 8);
-                    v[2 * s] = data[jj * LD + b];
-                    v[2 * s + 1] = cmul(data[(jj + ns) * LD + b], twiddle<SIGN>(tw, jj));
-                    dft2<SIGN>(v[2 * s], v[2 * s + 1]);
-                }
-            }
-            __syncthreads();
-            if (active) {
-#pragma unroll
-                for (int s = 0; s < 4; ++s) {
-                    const int jj = j + s * (N / 8);
-                    data[jj * LD + b] = v[2 * s];
-                    data[(jj + ns) * LD + b] = v[2 * s + 1];
-                }
-            }
-            __syncthreads();
-        }
-    }
 }
 
 // ---------------------------------------------------------------------------

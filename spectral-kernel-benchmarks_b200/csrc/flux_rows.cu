@@ -26,7 +26,7 @@
 #include "flux_rows.hpp"
 
 #include "async_copy.cuh"
-#include "fft_device.cuh"
+#include "fft_regs.cuh"
 #include "tensor_map.hpp"
 
 namespace skb {
@@ -270,50 +270,6 @@ __global__ void __launch_bounds__(32 * B, 16 / B) rows_flux_kernel(RowFluxArgs a
 // all transforms as in the warp-per-plane kernel, with one shared-memory
 // exchange per transform instead of two.  Lanes 0-15 own plane 2w of warp w,
 // lanes 16-31 plane 2w + 1.
-
-// Twiddle W16^e with exponent sign SIGN, e in {1, 2, 3, 6, 9} (e = 4 is a
-// multiplication by SIGN*i): cos(2 pi e / 16) + SIGN i sin(2 pi e / 16).
-template <int SIGN, int E>
-__device__ __forceinline__ float2 w16() {
-    constexpr float c1 = 0.923879532511286756128f;  // cos(pi/8)
-    constexpr float s1 = 0.382683432365089771728f;  // sin(pi/8)
-    constexpr float h = 0.707106781186547524401f;   // cos(pi/4)
-    constexpr float sg = SIGN < 0 ? -1.0f : 1.0f;
-    if constexpr (E == 1) return {c1, sg * s1};
-    if constexpr (E == 2) return {h, sg * h};
-    if constexpr (E == 3) return {s1, sg * c1};
-    if constexpr (E == 6) return {-h, sg * h};
-    return {-c1, -sg * s1};  // E == 9
-}
-
-// In-place length-16 DFT over v[0..15] (natural order in and out): 16 = 4 x 4,
-// input m = m2 + 4 m1, output k = k1 + 4 k2.
-template <int SIGN>
-__device__ __forceinline__ void dft16(float2 (&v)[16]) {
-#pragma unroll
-    for (int m2 = 0; m2 < 4; ++m2) dft4<SIGN>(v[m2], v[m2 + 4], v[m2 + 8], v[m2 + 12]);
-    // v[m2 + 4 k1] *= W16^(m2 k1)
-    v[5] = cmul(v[5], w16<SIGN, 1>());
-    v[9] = cmul(v[9], w16<SIGN, 2>());
-    v[13] = cmul(v[13], w16<SIGN, 3>());
-    v[6] = cmul(v[6], w16<SIGN, 2>());
-    v[10] = cmul_si<SIGN>(v[10]);
-    v[14] = cmul(v[14], w16<SIGN, 6>());
-    v[7] = cmul(v[7], w16<SIGN, 3>());
-    v[11] = cmul(v[11], w16<SIGN, 6>());
-    v[15] = cmul(v[15], w16<SIGN, 9>());
-#pragma unroll
-    for (int k1 = 0; k1 < 4; ++k1) dft4<SIGN>(v[4 * k1], v[4 * k1 + 1], v[4 * k1 + 2], v[4 * k1 + 3]);
-    // v[4 k1 + k2] holds output k1 + 4 k2: transpose the 4 x 4 block.
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = i + 1; j < 4; ++j) {
-            const float2 t = v[4 * i + j];
-            v[4 * i + j] = v[4 * j + i];
-            v[4 * j + i] = t;
-        }
-}
 
 // 256-point FFT of one half-warp's sequence: v[m] = z[t + 16 m] in, Z[t + 16 k]
 // in v[k] out.  xch: this half-warp's 16 x 17 exchange region; tw2[16 k2 + t] =

@@ -1,156 +1,336 @@
 // Horizontal transform kernels (row r2c/c2r along x, column c2c along y with
 // fused retention/embedding).  See horizontal.hpp for the decomposition and
-// fft_device.cuh for the shared-memory FFT.
+// fft_regs.cuh for the register-ended FFT.
 
 #include "horizontal.hpp"
 
-#include "fft_device.cuh"
+#include "fft_regs.cuh"
 
 namespace skb {
 namespace {
 
-// Batch width: 128-byte rows of complex values, capped so one CTA has at most
-// 1024 threads (fft_threads(N) * B <= 1024).
-template <typename T, int N>
-constexpr int batch_width() {
-    constexpr int natural = 128 / int(sizeof(cx<T>));
-    constexpr int cap = N >= 8 ? 8192 / N : 1024;
-    return natural < cap ? natural : cap;
+// Lanes of one shared-memory access phase (128 bytes of complex values): the
+// plane batch of a CTA is a multiple of it, so that global accesses along the
+// planes move whole 128-byte pieces.
+template <typename T>
+constexpr int phase_lanes() {
+    return 128 / int(sizeof(cx<T>));
 }
 
-template <typename T, int N>
-constexpr int cta_threads() {
-    return fft_threads(N) * batch_width<T, N>();
+// Resident CTAs per SM that a kernel is compiled for: what
+// shared memory, the registers it needs (per thread, by elements held) and the
+// thread limit allow.
+template <typename T>
+constexpr int resident_ctas(int threads, size_t bytes, int elements) {
+    const int regs = sizeof(T) == 8 ? (elements > 8 ? 96 : 64) : (elements > 8 ? 56 : 40);
+    int ctas = int(size_t(227 * 1024) / (bytes + 1024));
+    if (65536 / (threads * regs) < ctas) ctas = 65536 / (threads * regs);
+    if (2048 / threads < ctas) ctas = 2048 / threads;
+    return ctas < 1 ? 1 : ctas > 16 ? 16 : ctas;
 }
 
 // ---------------------------------------------------------------------------
+// Row kernels: M = Nx/2 complex points per row, B planes of one y per CTA.
+//
+// A row side and a plane side share the FFT.  On the row side T = M / E threads
+// (lanes of one warp) hold a row's elements t + T e, so that global accesses of
+// real rows run along x; on the plane side B consecutive lanes hold one bin of
+// B planes, so that global accesses of bins run along the planes.  The exchange
+// before the last pass (forward) or after the first one (inverse) is also the
+// turn from one side to the other: one shared-memory write and read per element
+// where a separate transpose tile took two more.  The plane side's radix-R pass
+// has Ns = M / R butterflies j over the bins j + Ns r; bin M - k of k = j + Ns r
+// belongs to butterfly Ns - j, so the real-spectrum split pairs butterflies
+// {j, Ns - j} in one thread's registers ({0, Ns/2} pair within themselves), or,
+// where a thread holds one butterfly only (M = 256), in two lanes that swap the
+// upper half of their values.
+//
+// Bound: latency, at 20 warps per SM (96 registers in FP64), then HBM.  FP64,
+// 516 planes of 512^2 kept to 171 bins (1.76 GB per launch): forward 426 ->
+// 301 us (5.9 TB/s), inverse 541 -> 354 us (5.0 TB/s) against the radix-8
+// kernels with every pass in shared memory; 195 planes of 256^2, all 129 bins:
+// 51 / 54 -> 37 / 39 us.  Persistent CTAs with the tables in shared memory and
+// the next tile's loads issued early ran 420 / 391 us, plane chunks sized for
+// L2 ran slower at every size (16 to 192 planes).
+template <typename T, int M>
+struct RowShape {
+    using V = cx<T>;
+    static constexpr int E = row_regs_per_thread(M);
+    static constexpr int TPR = M / E;  // row-side threads per row, at most 32
+    static constexpr int L = phase_lanes<T>();
+    static constexpr int B = TPR == 1 ? 32 : (128 / TPR > L) ? 128 / TPR : L;
+    static constexpr int NT = B * TPR;
+    static_assert(TPR <= 32 && E % 2 == 0 && B % L == 0, "a row's lanes form (part of) one warp");
+    static constexpr int R = row_plane_radix(M);
+    static constexpr int Ns = M / R;
+    static constexpr int NB = E / R;  // butterflies per plane-side thread
+    static constexpr size_t kBytes = TPR > 1 ? size_t(M) * B * sizeof(V) : 0;
+    static constexpr int kCtas = resident_ctas<T>(NT, kBytes, E);
+    // Position i of plane b in the exchange.  The swizzle spreads both sides'
+    // accesses over the banks: row lanes write positions E apart or walk
+    // consecutive ones (L / TPR planes per access phase when rows are short).
+    static constexpr int kMul = TPR < L ? L / TPR : 1;
+    static __device__ __forceinline__ int slot(int i, int b) { return i * B + (b ^ (((i ^ (i / E)) * kMul) & (L - 1))); }
+};
+
+// A row's own exchange among its lanes (512-point halves need two exchanges).
+template <typename S>
+struct RowExchange {
+    typename S::V* x;
+    int b;
+    __device__ __forceinline__ void store(int i, typename S::V v) { x[S::slot(i, b)] = v; }
+    __device__ __forceinline__ typename S::V load(int i) const { return x[S::slot(i, b)]; }
+    __device__ __forceinline__ void fence() const { __syncwarp(); }
+};
+
+// Butterfly of plane-side thread g when it holds one (M = 256): pairs
+// {j, 16 - j} in neighbouring groups of B lanes, 0 and 8 last.
+__device__ __forceinline__ int paired_butterfly(int g) {
+    const int h = g / 2 + 1;
+    return g >= 14 ? (g - 14) * 8 : (g & 1) ? 16 - h : h;
+}
+
+// Lane whose butterfly holds bin M - k (0 and 8: the lane itself).
+template <int B>
+__device__ __forceinline__ int pair_source(int j) {
+    const int lane = threadIdx.x & 31;
+    return (j & 7) == 0 ? lane : lane ^ B;
+}
+
 // Row forward: real rows of length NX = 2M -> bins kx in [0, keep).
 // Grid (plane chunks, ny).  The real row is read as M complex pairs
 // z[m] = x[2m] + i x[2m+1], transformed, then split into the real spectrum:
-//   X[k] = (Z[k] + conj Z[M-k])/2 - i/2 * W^k (Z[k] - conj Z[M-k]),  W = e^{-2 pi i/NX}.
+//   X[k] = s + W^k o,  X[M-k] = conj(s - W^k o),  W = e^{-2 pi i/NX},
+//   s = (Z[k] + conj Z[M-k])/2,  o = -i (Z[k] - conj Z[M-k])/2.
 template <typename T, int M>
-__global__ void __launch_bounds__(cta_threads<T, M>()) rows_forward_kernel(
-    int ny, long long planes, int keep, const T* __restrict__ real, DenseBins bins, const cx<T>* __restrict__ twHalf,
-    const cx<T>* __restrict__ twFull) {
+__global__ void __launch_bounds__(RowShape<T, M>::NT, RowShape<T, M>::kCtas)
+    rows_forward_kernel(int ny, long long planes, int keep, const T* __restrict__ real, DenseBins bins,
+                        const cx<T>* __restrict__ tw, const cx<T>* __restrict__ twFull) {
     using V = cx<T>;
-    constexpr int B = batch_width<T, M>();
-    constexpr int NT = cta_threads<T, M>();
-    extern __shared__ unsigned char smem_raw[];
+    using S = RowShape<T, M>;
+    constexpr int NX = 2 * M, R = S::R, Ns = S::Ns;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     V* data = reinterpret_cast<V*>(smem_raw);
     const int tid = threadIdx.x;
-    const long long p0 = (long long)blockIdx.x * B;
+    const long long p0 = (long long)blockIdx.x * S::B;
     const int y = blockIdx.y;
-    constexpr int NX = 2 * M;
-    constexpr int LD = B + 1;  // padded so the walk along x below is conflict-free
-    // Consecutive threads take consecutive x-pairs of one row: full-line loads,
-    // all of a thread's loads issued before the first shared store.
-    static_assert((M * B) % NT == 0, "whole load rounds");
+    V v[S::E];
+    {
+        const int t = tid % S::TPR;
+        const int b = tid / S::TPR;
+        if (p0 + b < planes) {
+            const V* row = reinterpret_cast<const V*>(real + ((p0 + b) * ny + y) * NX) + t;
 #pragma unroll
-    for (int it = 0; it < (M * B) / NT; ++it) {
-        const int idx = tid + it * NT;
-        const int m = idx % M;
-        const int b = idx / M;
-        const long long p = p0 + b;
-        V v = {T(0), T(0)};
-        if (p < planes) v = *reinterpret_cast<const V*>(real + (p * ny + y) * NX + 2 * m);
-        data[m * LD + b] = v;
-    }
-    __syncthreads();
-    fft_smem<T, M, B, -1, LD>(data, twHalf, tid, true);
-    V* out = reinterpret_cast<V*>(bins.data);
-    for (int idx = tid; idx < keep * B; idx += NT) {
-        const int b = idx % B;
-        const int k = idx / B;
-        const long long p = p0 + b;
-        if (p >= planes) continue;
-        V X;
-        const V z0 = data[b];
-        if (k == 0) {
-            X = {z0.x + z0.y, T(0)};
-        } else if (k == M) {
-            X = {z0.x - z0.y, T(0)};
+            for (int e = 0; e < S::E; ++e) v[e] = row[S::TPR * e];
         } else {
-            const V zk = data[k * LD + b];
-            const V zm = cconj(data[(M - k) * LD + b]);
-            const V e = cscale(cadd(zk, zm), T(0.5));
-            const V d = csub(zk, zm);
-            // o = -i/2 * d
-            const V o = {T(0.5) * d.y, T(-0.5) * d.x};
-            X = cadd(e, cmul(__ldg(twFull + k), o));
+#pragma unroll
+            for (int e = 0; e < S::E; ++e) v[e] = {T(0), T(0)};
         }
-        out[p + bins.planes * ((long long)k + bins.kxStride * y)] = X;
+        if constexpr (S::TPR > 1) {
+            RowExchange<S> xch{data, b};
+            fft_regs_head<T, M, S::E, -1, Ns>(v, t, tw, xch);
+            __syncthreads();
+        }
+    }
+    const int b = tid % S::B;
+    const int g = tid / S::B;
+    const bool live = p0 + b < planes;
+    const long long stride = bins.planes;
+    V* out = reinterpret_cast<V*>(bins.data) + bins.offset(live ? p0 + b : 0) + stride * bins.kxStride * y;
+    auto split = [&](int k, V zk, V zmk) {
+        const V zm = cconj(zmk);
+        const V s = cscale(cadd(zk, zm), T(0.5));
+        const V d = csub(zk, zm);
+        const V wo = cmul(__ldg(twFull + k), V{T(0.5) * d.y, T(-0.5) * d.x});
+        if (live && k < keep) out[stride * k] = cadd(s, wo);
+        if (live && 2 * k != M && M - k < keep) out[stride * (M - k)] = cconj(csub(s, wo));
+    };
+    auto split0 = [&](V z0) {
+        if (live) out[0] = {z0.x + z0.y, T(0)};
+        if (live && M < keep) out[stride * M] = {z0.x - z0.y, T(0)};
+    };
+    // Last pass of butterfly j: bins j + Ns r.
+    auto last = [&](int j, V* u) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) u[r] = data[S::slot(j + Ns * r, b)];
+        const V* w = tw + regs_table_offset(M, S::E, Ns) + j;
+#pragma unroll
+        for (int r = 1; r < R; ++r) u[r] = cmul(u[r], twiddle<-1>(w, Ns * (r - 1)));
+        dft_small<-1, R>(u);
+    };
+    if constexpr (S::TPR == 1) {
+        dft_small<-1, M>(v);
+        split0(v[0]);
+#pragma unroll
+        for (int k = 1; k <= M / 2; ++k) split(k, v[k], v[M - k]);
+    } else if constexpr (S::NB == 1) {
+        const int j = paired_butterfly(g);
+        const int src = pair_source<S::B>(j);
+        last(j, v);
+        const V half = v[R / 2];
+        if (j == 0) {
+            // Bin M - k of k = Ns r is register R - r: one up, like the other lanes'.
+#pragma unroll
+            for (int e = R / 2; e < R - 1; ++e) v[e] = v[e + 1];
+        }
+#pragma unroll
+        for (int r = 0; r < R / 2; ++r) {
+            const V other = {__shfl_sync(0xFFFFFFFFu, v[R - 1 - r].x, src), __shfl_sync(0xFFFFFFFFu, v[R - 1 - r].y, src)};
+            if (r > 0 || j > 0) split(j + Ns * r, v[r], other);
+        }
+        if (j == 0) {
+            split0(v[0]);
+            split(M / 2, half, half);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < S::NB / 2; ++i) {
+            const int q = g + S::TPR * i;
+            V a[R], c[R];
+            last(q, a);
+            last(q == 0 ? Ns / 2 : Ns - q, c);
+            if (i == 0 && q == 0) {
+                split0(a[0]);
+#pragma unroll
+                for (int r = 1; r <= R / 2; ++r) split(Ns * r, a[r], a[R - r]);
+#pragma unroll
+                for (int r = 0; r < R / 2; ++r) split(Ns / 2 + Ns * r, c[r], c[R - 1 - r]);
+            } else {
+#pragma unroll
+                for (int r = 0; r < R; ++r) split(q + Ns * r, a[r], c[R - 1 - r]);
+            }
+        }
     }
 }
 
 // Row inverse: bins kx in [0, keep) (zero above) -> real rows, unnormalised,
 // with FFTW's c2r semantics (imaginary parts of the kx = 0 and kx = NX/2 bins
-// are ignored).  Pre-process Z[k] = (X[k] + conj X[M-k]) + i e^{+2 pi i k/NX}
-// (X[k] - conj X[M-k]), then an inverse length-M FFT gives x[2m] + i x[2m+1].
+// are ignored).  Pre-process Z[k] = s + i t, Z[M-k] = conj(s - i t) with
+// s = X[k] + conj X[M-k], t = e^{+2 pi i k/NX} (X[k] - conj X[M-k]), then an
+// inverse length-M FFT gives x[2m] + i x[2m+1].  The radices run in the
+// forward kernel's order reversed, so the plane side has the same butterflies.
 template <typename T, int M>
-__global__ void __launch_bounds__(cta_threads<T, M>()) rows_inverse_kernel(
-    int ny, long long planes, int keep, DenseBins bins, T* __restrict__ real, const cx<T>* __restrict__ twHalf,
-    const cx<T>* __restrict__ twFull) {
+__global__ void __launch_bounds__(RowShape<T, M>::NT, RowShape<T, M>::kCtas)
+    rows_inverse_kernel(int ny, long long planes, int keep, DenseBins bins, T* __restrict__ real,
+                        const cx<T>* __restrict__ tw, const cx<T>* __restrict__ twFull) {
     using V = cx<T>;
-    constexpr int B = batch_width<T, M>();
-    constexpr int NT = cta_threads<T, M>();
-    extern __shared__ unsigned char smem_raw[];
+    using S = RowShape<T, M>;
+    constexpr int NX = 2 * M, R = S::R, Ns = S::Ns;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     V* data = reinterpret_cast<V*>(smem_raw);
     const int tid = threadIdx.x;
-    const long long p0 = (long long)blockIdx.x * B;
+    const long long p0 = (long long)blockIdx.x * S::B;
     const int y = blockIdx.y;
-    constexpr int NX = 2 * M;
-    constexpr int LD = B + 1;
-    const V* in = reinterpret_cast<const V*>(bins.data);
-    auto load = [&](int k, int b) -> V {
-        const long long p = p0 + b;
-        if (k >= keep || p >= planes) return V{T(0), T(0)};
-        V v = in[p + bins.planes * ((long long)k + bins.kxStride * y)];
-        if (k == 0 || k == M) v.y = T(0);
-        return v;
-    };
-    // Pairs (k, M-k) for k in [0, M/2]; k = 0 pairs with the Nyquist bin M.
-    constexpr int pairs = M / 2 + 1;
-    // FP64 issues all of a thread's loads first; FP32 measured faster rolled.
-    constexpr int kUnroll = sizeof(T) == 8 ? (pairs * B + NT - 1) / NT : 1;
-#pragma unroll kUnroll
-    for (int it = 0; it < (pairs * B + NT - 1) / NT; ++it) {
-        const int idx = tid + it * NT;
-        if (idx >= pairs * B) break;
-        const int b = idx % B;
-        const int k = idx / B;
-        if (k == 0) {
-            const V x0 = load(0, b);
-            const V xm = load(M, b);
-            data[b] = {x0.x + xm.x, x0.x - xm.x};
-            continue;
-        }
-        const int kk = M - k;
-        const V xk = load(k, b);
-        const V xm = load(kk, b);
-        {
+    V v[S::E];
+    {
+        const int b = tid % S::B;
+        const int g = tid / S::B;
+        const bool live = p0 + b < planes;
+        const long long stride = bins.planes;
+        const V* in =
+            reinterpret_cast<const V*>(bins.data) + bins.offset(live ? p0 + b : 0) + stride * bins.kxStride * y;
+        auto load = [&](int k) -> V { return live && k < keep ? in[stride * k] : V{T(0), T(0)}; };
+        // (X[k], X[M-k]) -> (Z[k], Z[M-k])
+        auto merge = [&](int k, V& xk, V& xm) {
             const V s = cadd(xk, cconj(xm));
-            const V d = csub(xk, cconj(xm));
-            const V t = cmulc(d, __ldg(twFull + k));  // d * e^{+2 pi i k/NX}
-            data[k * LD + b] = {s.x - t.y, s.y + t.x};   // s + i t
-        }
-        if (kk != k) {
-            const V s = cadd(xm, cconj(xk));
-            const V d = csub(xm, cconj(xk));
-            const V t = cmulc(d, __ldg(twFull + kk));
-            data[kk * LD + b] = {s.x - t.y, s.y + t.x};
-        }
-    }
-    __syncthreads();
-    fft_smem<T, M, B, +1, LD>(data, twHalf, tid, true);
-    // Consecutive threads write consecutive x-pairs of one row.
+            const V w = cmulc(csub(xk, cconj(xm)), __ldg(twFull + k));
+            xk = {s.x - w.y, s.y + w.x};
+            xm = {s.x + w.y, w.x - s.y};
+        };
+        // Bins 0 and NX/2 are real.
+        auto merge0 = [&](V& x0, V xn) { x0 = {x0.x + xn.x, x0.x - xn.x}; };
+        // First pass of butterfly j (positions j R + r of the exchange).
+        auto first = [&](int j, V* u) {
+            dft_small<+1, R>(u);
 #pragma unroll
-    for (int it = 0; it < (M * B) / NT; ++it) {
-        const int idx = tid + it * NT;
-        const int m = idx % M;
-        const int b = idx / M;
-        const long long p = p0 + b;
-        if (p < planes) *reinterpret_cast<V*>(real + (p * ny + y) * NX + 2 * m) = data[m * LD + b];
+            for (int r = 0; r < R; ++r) data[S::slot(j * R + r, b)] = u[r];
+        };
+        if constexpr (S::TPR == 1) {
+#pragma unroll
+            for (int k = 0; k < M; ++k) v[k] = load(k);
+            merge0(v[0], load(M));
+#pragma unroll
+            for (int k = 1; k <= M / 2; ++k) {
+                V xm = v[M - k];
+                merge(k, v[k], xm);
+                if (2 * k != M) v[M - k] = xm;
+            }
+            dft_small<+1, M>(v);
+        } else if constexpr (S::NB == 1) {
+            const int j = paired_butterfly(g);
+            const int src = pair_source<S::B>(j);
+            // Butterfly 0 holds the partners one register up: its upper half is
+            // loaded (and put back) shifted, bin NX/2 last, bin M/2 apart.
+            V half = j == 0 ? load(M / 2) : V{T(0), T(0)};
+#pragma unroll
+            for (int r = 0; r < R; ++r) v[r] = load(j + Ns * r + (r >= R / 2 && j == 0 ? Ns : 0));
+#pragma unroll
+            for (int r = 0; r < R / 2; ++r) {
+                V& up = v[R - 1 - r];
+                V other = {__shfl_sync(0xFFFFFFFFu, up.x, src), __shfl_sync(0xFFFFFFFFu, up.y, src)};
+                if (r == 0 && j == 0)
+                    merge0(v[0], other);
+                else
+                    merge(j + Ns * r, v[r], other);
+                // Z[M-k] goes back to the lane that X[M-k] came from.
+                up = {__shfl_sync(0xFFFFFFFFu, other.x, src), __shfl_sync(0xFFFFFFFFu, other.y, src)};
+            }
+            if (j == 0) {
+                V self = half;
+                merge(M / 2, half, self);
+#pragma unroll
+                for (int e = R - 1; e > R / 2; --e) v[e] = v[e - 1];
+                v[R / 2] = half;
+            }
+            first(j, v);
+        } else {
+#pragma unroll
+            for (int i = 0; i < S::NB / 2; ++i) {
+                const int q = g + S::TPR * i;
+                const int qc = q == 0 ? Ns / 2 : Ns - q;
+                V* a = v + 2 * R * i;
+                V* c = a + R;
+#pragma unroll
+                for (int r = 0; r < R; ++r) a[r] = load(q + Ns * r);
+#pragma unroll
+                for (int r = 0; r < R; ++r) c[r] = load(qc + Ns * r);
+            }
+#pragma unroll
+            for (int i = 0; i < S::NB / 2; ++i) {
+                const int q = g + S::TPR * i;
+                const int qc = q == 0 ? Ns / 2 : Ns - q;
+                V* a = v + 2 * R * i;
+                V* c = a + R;
+                if (i == 0 && q == 0) {
+                    merge0(a[0], load(M));
+#pragma unroll
+                    for (int r = 1; r < R / 2; ++r) merge(Ns * r, a[r], a[R - r]);
+                    V self = a[R / 2];
+                    merge(M / 2, a[R / 2], self);
+#pragma unroll
+                    for (int r = 0; r < R / 2; ++r) merge(Ns / 2 + Ns * r, c[r], c[R - 1 - r]);
+                } else {
+#pragma unroll
+                    for (int r = 0; r < R; ++r) merge(q + Ns * r, a[r], c[R - 1 - r]);
+                }
+                first(q, a);
+                first(qc, c);
+            }
+        }
     }
+    const int t = tid % S::TPR;
+    const int b = tid / S::TPR;
+    if constexpr (S::TPR > 1) {
+        __syncthreads();
+        RowExchange<S> xch{data, b};
+#pragma unroll
+        for (int e = 0; e < S::E; ++e) v[e] = xch.load(t + S::TPR * e);
+        fft_regs<T, M, S::E, +1, R>(v, t, tw, xch);
+    }
+    if (p0 + b >= planes) return;
+    V* row = reinterpret_cast<V*>(real + ((p0 + b) * ny + y) * NX) + t;
+#pragma unroll
+    for (int e = 0; e < S::E; ++e) row[S::TPR * e] = v[e];
 }
 
 // Length-1 rows (Nx = 2): X[0] = x0 + x1, X[1] = x0 - x1.
@@ -162,14 +342,14 @@ __global__ void rows_pair_kernel(int dir, int ny, long long planes, int keep, co
     if (i >= planes * ny) return;
     const long long p = i % planes;
     const long long y = i / planes;
-    V* b = reinterpret_cast<V*>(bins.data);
+    V* b = reinterpret_cast<V*>(bins.data) + bins.offset(p);
     if (dir < 0) {
         const T x0 = realIn[(p * ny + y) * 2], x1 = realIn[(p * ny + y) * 2 + 1];
-        b[p + bins.planes * (0 + bins.kxStride * y)] = {x0 + x1, T(0)};
-        if (keep > 1) b[p + bins.planes * (1 + bins.kxStride * y)] = {x0 - x1, T(0)};
+        b[bins.planes * (0 + bins.kxStride * y)] = {x0 + x1, T(0)};
+        if (keep > 1) b[bins.planes * (1 + bins.kxStride * y)] = {x0 - x1, T(0)};
     } else {
-        const T a = b[p + bins.planes * (0 + bins.kxStride * y)].x;
-        const T c = keep > 1 ? b[p + bins.planes * (1 + bins.kxStride * y)].x : T(0);
+        const T a = b[bins.planes * (0 + bins.kxStride * y)].x;
+        const T c = keep > 1 ? b[bins.planes * (1 + bins.kxStride * y)].x : T(0);
         realOut[(p * ny + y) * 2] = a + c;
         realOut[(p * ny + y) * 2 + 1] = a - c;
     }
@@ -196,135 +376,95 @@ __device__ __forceinline__ void view_store(const FieldView& v, long long mode, i
     }
 }
 
-template <typename T, int N, int SIGN>
-__global__ void __launch_bounds__(cta_threads<T, N>()) columns_dense_kernel(long long planes, DenseBins in,
-                                                                            DenseBins out,
-                                                                            const cx<T>* __restrict__ tw) {
+// Column kernels: tiles of one kx column of N points for B = L planes (128-byte
+// pieces of every ky row); threads (plane b, t) with b fastest, so each
+// exchange access is a run of L consecutive values, free of bank conflicts at
+// any stride.  Elements go from HBM to registers and back: one exchange (two
+// above 256 points) is the only shared-memory traffic.  Grid (plane chunks, kx).
+// Bound: latency (load waits at 20-30 warps per SM), then HBM.  FP64: 512-point
+// embedding / retention of 516 planes (1.1 GB) 436 / 358 -> 301 / 234 us, dense
+// 256-point columns of 195 planes (205 MB) 49 -> 42 us; half as many planes
+// per CTA moved the first two to 280 / 258 us, persistent CTAs to 329 / 289 us.
+template <typename T, int N>
+struct ColumnShape {
     using V = cx<T>;
-    constexpr int B = batch_width<T, N>();
-    constexpr int NT = cta_threads<T, N>();
-    extern __shared__ unsigned char smem_raw[];
-    V* data = reinterpret_cast<V*>(smem_raw);
-    const int tid = threadIdx.x;
-    const long long p0 = (long long)blockIdx.x * B;
+    static constexpr int E = column_regs_per_thread(N, sizeof(T) == 8);
+    static constexpr int TPC = N / E;
+    static constexpr int B = phase_lanes<T>();
+    static constexpr int NT = B * TPC;
+    static constexpr size_t kBytes = TPC > 1 ? size_t(N) * B * sizeof(V) : 0;
+    static constexpr int kCtas = resident_ctas<T>(NT, kBytes, E);
+};
+
+template <typename V, int B>
+struct ColumnExchange {
+    V* x;  // this thread's plane of [position][plane]
+    __device__ __forceinline__ void store(int i, V v) { x[i * B] = v; }
+    __device__ __forceinline__ V load(int i) const { return x[i * B]; }
+    __device__ __forceinline__ void fence() const { __syncthreads(); }
+};
+
+// Input and output of a column kernel: plane p of a dense bin array, or level
+// p mod nz of retained view p / nz, so that chunks of planes run on across
+// views and only the last one is ragged.
+enum class ColumnIo { dense, views };
+
+template <typename T, int N, int SIGN, ColumnIo IN, ColumnIo OUT>
+__global__ void __launch_bounds__(ColumnShape<T, N>::NT, ColumnShape<T, N>::kCtas)
+    columns_kernel(long long planes, DenseBins in, DenseBins out, int nz,
+                   const __grid_constant__ ViewSet views, const int* __restrict__ cells, T scale,
+                   const cx<T>* __restrict__ tw) {
+    using V = cx<T>;
+    using S = ColumnShape<T, N>;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int b = threadIdx.x % S::B;
+    const int t = threadIdx.x / S::B;
+    ColumnExchange<V, S::B> xch{reinterpret_cast<V*>(smem_raw) + b};
     const long long kx = blockIdx.y;
-    const V* src = reinterpret_cast<const V*>(in.data);
-    static_assert((N * B) % NT == 0, "whole load rounds");
-#pragma unroll
-    for (int it = 0; it < (N * B) / NT; ++it) {
-        const int idx = tid + it * NT;
-        const int b = idx % B;
-        const int ky = idx / B;
-        const long long p = p0 + b;
-        V v = {T(0), T(0)};
-        if (p < planes) v = src[p + in.planes * (kx + in.kxStride * ky)];
-        data[ky * B + b] = v;
+    const long long p = (long long)blockIdx.x * S::B + b;
+    const bool live = p < planes;
+    FieldView view{};
+    int z = 0;
+    if (IN == ColumnIo::views || OUT == ColumnIo::views) {
+        const int f = live ? int(p / nz) : 0;
+        z = live ? int(p - (long long)f * nz) : 0;
+        view = views.v[f];
     }
-    __syncthreads();
-    fft_smem<T, N, B, SIGN>(data, tw, tid, true);
-    V* dst = reinterpret_cast<V*>(out.data);
+    const int* map = cells + kx * N + t;
+    V v[S::E];
+    if constexpr (IN == ColumnIo::views) {
+        int cell[S::E];
 #pragma unroll
-    for (int it = 0; it < (N * B) / NT; ++it) {
-        const int idx = tid + it * NT;
-        const int b = idx % B;
-        const int ky = idx / B;
-        const long long p = p0 + b;
-        if (p < planes) dst[p + out.planes * (kx + out.kxStride * ky)] = data[ky * B + b];
+        for (int e = 0; e < S::E; ++e) cell[e] = __ldg(map + S::TPC * e);
+#pragma unroll
+        for (int e = 0; e < S::E; ++e)
+            v[e] = live && cell[e] >= 0 ? view_load<T>(view, cell[e] >> 1, z) : V{T(0), T(0)};
+#pragma unroll
+        for (int e = 0; e < S::E; ++e)
+            if (cell[e] & 1) v[e] = cconj(v[e]);
+    } else {
+        const V* src =
+            reinterpret_cast<const V*>(in.data) + in.offset(live ? p : 0) + in.planes * (kx + in.kxStride * t);
+        const long long step = in.planes * in.kxStride * S::TPC;
+#pragma unroll
+        for (int e = 0; e < S::E; ++e) v[e] = live ? src[step * e] : V{T(0), T(0)};
     }
-}
-
-// Inverse column with retained-mode input: chunk c covers view f = c / zChunks,
-// z in [z0, z0+B).  Dense output plane index = f*nz + z.
-template <typename T, int N>
-__global__ void __launch_bounds__(cta_threads<T, N>()) columns_embed_kernel(int nz, ViewSet views, ModeTables tables,
-                                                                            DenseBins out,
-                                                                            const cx<T>* __restrict__ tw) {
-    using V = cx<T>;
-    constexpr int B = batch_width<T, N>();
-    constexpr int NT = cta_threads<T, N>();
-    extern __shared__ unsigned char smem_raw[];
-    V* data = reinterpret_cast<V*>(smem_raw);
-    const int tid = threadIdx.x;
-    const int zChunks = (nz + B - 1) / B;
-    const int f = blockIdx.x / zChunks;
-    const int z0 = (blockIdx.x % zChunks) * B;
-    const int kx = blockIdx.y;
-    const FieldView view = views.v[f];
-    const int* map = tables.cellMap + (long long)kx * N;
-    static_assert((N * B) % NT == 0, "whole load rounds");
-    // FP64 issues all of a thread's loads first; FP32 measured faster rolled.
-    constexpr int kUnroll = sizeof(T) == 8 ? (N * B) / NT : 1;
-#pragma unroll kUnroll
-    for (int it = 0; it < (N * B) / NT; ++it) {
-        const int idx = tid + it * NT;
-        const int b = idx % B;
-        const int ky = idx / B;
-        const int z = z0 + b;
-        V v = {T(0), T(0)};
-        const int e = __ldg(map + ky);
-        if (e >= 0 && z < nz) {
-            v = view_load<T>(view, e >> 1, z);
-            if (e & 1) v = cconj(v);
+    fft_regs<T, N, S::E, SIGN>(v, t, tw, xch);
+    if (!live) return;
+    if constexpr (OUT == ColumnIo::views) {
+#pragma unroll
+        for (int e = 0; e < S::E; ++e) {
+            const int cell = __ldg(map + S::TPC * e);
+            if (cell < 0) continue;
+            V x = cscale(v[e], scale);
+            if (cell & 1) x = cconj(x);
+            view_store<T>(view, cell >> 1, z, x);
         }
-        data[ky * B + b] = v;
-    }
-    __syncthreads();
-    fft_smem<T, N, B, +1>(data, tw, tid, true);
-    V* dst = reinterpret_cast<V*>(out.data);
-    const long long pBase = (long long)f * nz;
+    } else {
+        V* dst = reinterpret_cast<V*>(out.data) + out.offset(p) + out.planes * (kx + out.kxStride * t);
+        const long long step = out.planes * out.kxStride * S::TPC;
 #pragma unroll
-    for (int it = 0; it < (N * B) / NT; ++it) {
-        const int idx = tid + it * NT;
-        const int b = idx % B;
-        const int ky = idx / B;
-        const int z = z0 + b;
-        if (z < nz) dst[pBase + z + out.planes * (kx + out.kxStride * ky)] = data[ky * B + b];
-    }
-}
-
-// Forward column with retained-mode output.
-template <typename T, int N>
-__global__ void __launch_bounds__(cta_threads<T, N>()) columns_gather_kernel(int nz, DenseBins in, ViewSet views,
-                                                                             ModeTables tables, T scale,
-                                                                             const cx<T>* __restrict__ tw) {
-    using V = cx<T>;
-    constexpr int B = batch_width<T, N>();
-    constexpr int NT = cta_threads<T, N>();
-    extern __shared__ unsigned char smem_raw[];
-    V* data = reinterpret_cast<V*>(smem_raw);
-    const int tid = threadIdx.x;
-    const int zChunks = (nz + B - 1) / B;
-    const int f = blockIdx.x / zChunks;
-    const int z0 = (blockIdx.x % zChunks) * B;
-    const int kx = blockIdx.y;
-    const V* src = reinterpret_cast<const V*>(in.data);
-    const long long pBase = (long long)f * nz;
-    static_assert((N * B) % NT == 0, "whole load rounds");
-#pragma unroll
-    for (int it = 0; it < (N * B) / NT; ++it) {
-        const int idx = tid + it * NT;
-        const int b = idx % B;
-        const int ky = idx / B;
-        const int z = z0 + b;
-        V v = {T(0), T(0)};
-        if (z < nz) v = src[pBase + z + in.planes * ((long long)kx + in.kxStride * ky)];
-        data[ky * B + b] = v;
-    }
-    __syncthreads();
-    fft_smem<T, N, B, -1>(data, tw, tid, true);
-    const FieldView view = views.v[f];
-    const int begin = __ldg(tables.colStart + kx);
-    const int end = __ldg(tables.colStart + kx + 1);
-    for (int idx = tid; idx < (end - begin) * B; idx += NT) {
-        const int b = idx % B;
-        const int e = begin + idx / B;
-        const int z = z0 + b;
-        if (z >= nz) continue;
-        const int ky = __ldg(tables.colKy + e);
-        const int mc = __ldg(tables.colMode + e);
-        V v = cscale(data[ky * B + b], scale);
-        if (mc & 1) v = cconj(v);
-        view_store<T>(view, mc >> 1, z, v);
+        for (int e = 0; e < S::E; ++e) dst[step * e] = v[e];
     }
 }
 
@@ -369,36 +509,38 @@ __global__ void embed_dense_kernel(int ny, int nz, ViewSet views, ModeTables tab
 // ---------------------------------------------------------------------------
 // Dispatch helpers.
 
-template <typename T, int N>
-size_t smem_bytes() {
-    return size_t(N) * batch_width<T, N>() * sizeof(cx<T>);
-}
-
-// Row kernels pad each shared row by one element (stride B + 1).
-template <typename T, int N>
-size_t row_smem_bytes() {
-    return size_t(N) * (batch_width<T, N>() + 1) * sizeof(cx<T>);
-}
-
 template <typename K>
 cudaError_t allow_smem(K kernel, size_t bytes) {
     if (bytes <= 48 * 1024) return cudaSuccess;
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
 }
 
-#define SKB_LENGTH_SWITCH(n, ...)       \
-    switch (n) {                        \
-        case 2: { constexpr int L = 2; __VA_ARGS__; } break;       \
-        case 4: { constexpr int L = 4; __VA_ARGS__; } break;       \
-        case 8: { constexpr int L = 8; __VA_ARGS__; } break;       \
-        case 16: { constexpr int L = 16; __VA_ARGS__; } break;     \
-        case 32: { constexpr int L = 32; __VA_ARGS__; } break;     \
-        case 64: { constexpr int L = 64; __VA_ARGS__; } break;     \
-        case 128: { constexpr int L = 128; __VA_ARGS__; } break;   \
-        case 256: { constexpr int L = 256; __VA_ARGS__; } break;   \
-        case 512: { constexpr int L = 512; __VA_ARGS__; } break;   \
-        case 1024: { constexpr int L = 1024; __VA_ARGS__; } break; \
-        default: return cudaErrorInvalidValue;              \
+#define SKB_LENGTH_CASE(n, ...) \
+    case n: {                   \
+        constexpr int L = n;    \
+        __VA_ARGS__;            \
+    } break;
+// Half row lengths (Nx / 2) up to 512; column lengths reach 1024.
+#define SKB_HALF_CASES(...)         \
+    SKB_LENGTH_CASE(2, __VA_ARGS__)   \
+    SKB_LENGTH_CASE(4, __VA_ARGS__)   \
+    SKB_LENGTH_CASE(8, __VA_ARGS__)   \
+    SKB_LENGTH_CASE(16, __VA_ARGS__)  \
+    SKB_LENGTH_CASE(32, __VA_ARGS__)  \
+    SKB_LENGTH_CASE(64, __VA_ARGS__)  \
+    SKB_LENGTH_CASE(128, __VA_ARGS__) \
+    SKB_LENGTH_CASE(256, __VA_ARGS__) \
+    SKB_LENGTH_CASE(512, __VA_ARGS__)
+#define SKB_HALF_SWITCH(n, ...)                   \
+    switch (n) {                                  \
+        SKB_HALF_CASES(__VA_ARGS__)               \
+        default: return cudaErrorInvalidValue;    \
+    }
+#define SKB_LENGTH_SWITCH(n, ...)                 \
+    switch (n) {                                  \
+        SKB_HALF_CASES(__VA_ARGS__)               \
+        SKB_LENGTH_CASE(1024, __VA_ARGS__)        \
+        default: return cudaErrorInvalidValue;    \
     }
 
 template <typename T>
@@ -411,16 +553,15 @@ cudaError_t rows_forward_t(int nx, int ny, long long planes, int keep, const voi
                                                                             static_cast<const T*>(real), nullptr, bins);
         return cudaGetLastError();
     }
-    SKB_LENGTH_SWITCH(M, {
-        constexpr int B = batch_width<T, L>();
+    SKB_HALF_SWITCH(M, {
+        using S = RowShape<T, L>;
         auto kernel = rows_forward_kernel<T, L>;
-        const size_t bytes = row_smem_bytes<T, L>();
-        cudaError_t err = allow_smem(kernel, bytes);
+        const cudaError_t err = allow_smem(kernel, S::kBytes);
         if (err != cudaSuccess) return err;
-        dim3 grid(unsigned((planes + B - 1) / B), unsigned(ny));
-        kernel<<<grid, cta_threads<T, L>(), bytes, stream>>>(ny, planes, keep, static_cast<const T*>(real), bins,
-                                                             static_cast<const cx<T>*>(twHalf),
-                                                             static_cast<const cx<T>*>(twFull));
+        const dim3 grid(unsigned((planes + S::B - 1) / S::B), unsigned(ny));
+        kernel<<<grid, S::NT, S::kBytes, stream>>>(ny, planes, keep, static_cast<const T*>(real), bins,
+                                                   static_cast<const cx<T>*>(twHalf),
+                                                   static_cast<const cx<T>*>(twFull));
     });
     return cudaGetLastError();
 }
@@ -435,74 +576,35 @@ cudaError_t rows_inverse_t(int nx, int ny, long long planes, int keep, DenseBins
                                                                             static_cast<T*>(real), bins);
         return cudaGetLastError();
     }
-    SKB_LENGTH_SWITCH(M, {
-        constexpr int B = batch_width<T, L>();
+    SKB_HALF_SWITCH(M, {
+        using S = RowShape<T, L>;
         auto kernel = rows_inverse_kernel<T, L>;
-        const size_t bytes = row_smem_bytes<T, L>();
-        cudaError_t err = allow_smem(kernel, bytes);
+        const cudaError_t err = allow_smem(kernel, S::kBytes);
         if (err != cudaSuccess) return err;
-        dim3 grid(unsigned((planes + B - 1) / B), unsigned(ny));
-        kernel<<<grid, cta_threads<T, L>(), bytes, stream>>>(ny, planes, keep, bins, static_cast<T*>(real),
-                                                             static_cast<const cx<T>*>(twHalf),
-                                                             static_cast<const cx<T>*>(twFull));
+        const dim3 grid(unsigned((planes + S::B - 1) / S::B), unsigned(ny));
+        kernel<<<grid, S::NT, S::kBytes, stream>>>(ny, planes, keep, bins, static_cast<T*>(real),
+                                                   static_cast<const cx<T>*>(twHalf),
+                                                   static_cast<const cx<T>*>(twFull));
     });
     return cudaGetLastError();
 }
 
-template <typename T>
-cudaError_t columns_dense_t(int sign, int ny, int columns, long long planes, DenseBins in, DenseBins out,
-                            const void* tw, cudaStream_t stream) {
+template <typename T, int SIGN, ColumnIo IN, ColumnIo OUT>
+cudaError_t columns_t(int ny, int columns, long long planes, DenseBins in, DenseBins out, int nz, const ViewSet& views,
+                      const int* cells, double scale, const void* tw, cudaStream_t stream) {
     SKB_LENGTH_SWITCH(ny, {
-        constexpr int B = batch_width<T, L>();
-        const size_t bytes = smem_bytes<T, L>();
-        dim3 grid(unsigned((planes + B - 1) / B), unsigned(columns));
-        if (sign < 0) {
-            auto kernel = columns_dense_kernel<T, L, -1>;
-            cudaError_t err = allow_smem(kernel, bytes);
-            if (err != cudaSuccess) return err;
-            kernel<<<grid, cta_threads<T, L>(), bytes, stream>>>(planes, in, out, static_cast<const cx<T>*>(tw));
-        } else {
-            auto kernel = columns_dense_kernel<T, L, +1>;
-            cudaError_t err = allow_smem(kernel, bytes);
-            if (err != cudaSuccess) return err;
-            kernel<<<grid, cta_threads<T, L>(), bytes, stream>>>(planes, in, out, static_cast<const cx<T>*>(tw));
-        }
+        using S = ColumnShape<T, L>;
+        auto kernel = columns_kernel<T, L, SIGN, IN, OUT>;
+        const cudaError_t err = allow_smem(kernel, S::kBytes);
+        if (err != cudaSuccess) return err;
+        const dim3 grid(unsigned((planes + S::B - 1) / S::B), unsigned(columns));
+        kernel<<<grid, S::NT, S::kBytes, stream>>>(planes, in, out, nz, views, cells, T(scale),
+                                                   static_cast<const cx<T>*>(tw));
     });
     return cudaGetLastError();
 }
 
-template <typename T>
-cudaError_t columns_embed_t(int ny, int nz, int columns, const ViewSet& views, const ModeTables& tables,
-                            DenseBins out, const void* tw, cudaStream_t stream) {
-    SKB_LENGTH_SWITCH(ny, {
-        constexpr int B = batch_width<T, L>();
-        const size_t bytes = smem_bytes<T, L>();
-        auto kernel = columns_embed_kernel<T, L>;
-        cudaError_t err = allow_smem(kernel, bytes);
-        if (err != cudaSuccess) return err;
-        const int zChunks = (nz + B - 1) / B;
-        dim3 grid(unsigned(zChunks * views.count), unsigned(columns));
-        kernel<<<grid, cta_threads<T, L>(), bytes, stream>>>(nz, views, tables, out, static_cast<const cx<T>*>(tw));
-    });
-    return cudaGetLastError();
-}
-
-template <typename T>
-cudaError_t columns_gather_t(int ny, int nz, int columns, DenseBins in, const ViewSet& views,
-                             const ModeTables& tables, double scale, const void* tw, cudaStream_t stream) {
-    SKB_LENGTH_SWITCH(ny, {
-        constexpr int B = batch_width<T, L>();
-        const size_t bytes = smem_bytes<T, L>();
-        auto kernel = columns_gather_kernel<T, L>;
-        cudaError_t err = allow_smem(kernel, bytes);
-        if (err != cudaSuccess) return err;
-        const int zChunks = (nz + B - 1) / B;
-        dim3 grid(unsigned(zChunks * views.count), unsigned(columns));
-        kernel<<<grid, cta_threads<T, L>(), bytes, stream>>>(nz, in, views, tables, T(scale),
-                                                             static_cast<const cx<T>*>(tw));
-    });
-    return cudaGetLastError();
-}
+const ViewSet kNoViews{};
 
 }  // namespace
 
@@ -525,22 +627,32 @@ cudaError_t launch_rows_inverse(Precision p, int nx, int ny, long long planes, i
 cudaError_t launch_columns_dense(Precision p, int sign, int ny, int columns, long long planes, DenseBins in,
                                  DenseBins out, const void* tw, cudaStream_t stream) {
     if (planes <= 0 || columns <= 0) return cudaSuccess;
-    return p == Precision::f64 ? columns_dense_t<double>(sign, ny, columns, planes, in, out, tw, stream)
-                               : columns_dense_t<float>(sign, ny, columns, planes, in, out, tw, stream);
+    constexpr auto D = ColumnIo::dense;
+    if (p == Precision::f64)
+        return sign < 0 ? columns_t<double, -1, D, D>(ny, columns, planes, in, out, 1, kNoViews, nullptr, 1.0, tw, stream)
+                        : columns_t<double, +1, D, D>(ny, columns, planes, in, out, 1, kNoViews, nullptr, 1.0, tw, stream);
+    return sign < 0 ? columns_t<float, -1, D, D>(ny, columns, planes, in, out, 1, kNoViews, nullptr, 1.0, tw, stream)
+                    : columns_t<float, +1, D, D>(ny, columns, planes, in, out, 1, kNoViews, nullptr, 1.0, tw, stream);
 }
 
 cudaError_t launch_columns_embed(Precision p, int ny, int nz, int columns, const ViewSet& views,
                                  const ModeTables& tables, DenseBins out, const void* tw, cudaStream_t stream) {
     if (views.count <= 0 || columns <= 0) return cudaSuccess;
-    return p == Precision::f64 ? columns_embed_t<double>(ny, nz, columns, views, tables, out, tw, stream)
-                               : columns_embed_t<float>(ny, nz, columns, views, tables, out, tw, stream);
+    constexpr auto D = ColumnIo::dense, W = ColumnIo::views;
+    const long long planes = (long long)nz * views.count;
+    return p == Precision::f64
+               ? columns_t<double, +1, W, D>(ny, columns, planes, {}, out, nz, views, tables.cellMap, 1.0, tw, stream)
+               : columns_t<float, +1, W, D>(ny, columns, planes, {}, out, nz, views, tables.cellMap, 1.0, tw, stream);
 }
 
 cudaError_t launch_columns_gather(Precision p, int ny, int nz, int columns, DenseBins in, const ViewSet& views,
                                   const ModeTables& tables, double scale, const void* tw, cudaStream_t stream) {
     if (views.count <= 0 || columns <= 0) return cudaSuccess;
-    return p == Precision::f64 ? columns_gather_t<double>(ny, nz, columns, in, views, tables, scale, tw, stream)
-                               : columns_gather_t<float>(ny, nz, columns, in, views, tables, scale, tw, stream);
+    constexpr auto D = ColumnIo::dense, W = ColumnIo::views;
+    const long long planes = (long long)nz * views.count;
+    return p == Precision::f64
+               ? columns_t<double, -1, D, W>(ny, columns, planes, in, {}, nz, views, tables.gatherMap, scale, tw, stream)
+               : columns_t<float, -1, D, W>(ny, columns, planes, in, {}, nz, views, tables.gatherMap, scale, tw, stream);
 }
 
 cudaError_t launch_gather_dense(Precision p, int ny, int nz, long long modes, const int* modeKx, const int* modeKy,

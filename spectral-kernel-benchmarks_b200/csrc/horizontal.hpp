@@ -52,12 +52,61 @@ enum class Precision { f64 = 0, f32 = 1 };
 
 struct DenseBins {
     void* data;          // complex T
-    long long planes;    // stride between consecutive kx (total planes)
+    long long planes;    // stride between consecutive kx (total planes, or planes of a block)
     long long kxStride;  // number of kx entries per ky row
+    // Plane-blocked arrays (the plans' scratch): blocks of 2^blockShift planes,
+    // each a [ky][kx][plane of the block] array of blockStride elements.
+    int blockShift = 0;
+    long long blockStride = 0;  // 0: one array, all planes innermost
+    __host__ __device__ long long offset(long long plane) const {
+        if (blockStride == 0) return plane;
+        const long long block = plane >> blockShift;
+        return block * blockStride + (plane - (block << blockShift));
+    }
 };
 
+// Elements of a length-n sequence that one thread of the register-ended FFT
+// holds (fft_regs.cuh).  Lengths up to 16 stay in one thread; 16 elements make
+// 128- and 256-point transforms one exchange.  FP64 512-point columns hold 8:
+// 16 would need twice the registers for the same two exchanges.
+constexpr int regs_per_thread(int n) { return n <= 16 ? n : n <= 64 ? 8 : 16; }
+constexpr int column_regs_per_thread(int n, bool f64) { return n == 512 && f64 ? 8 : regs_per_thread(n); }
+// Row kernels (half-length m = Nx/2): elements per thread and the radix of the
+// pass that runs along the planes.
+constexpr int row_regs_per_thread(int m) { return m <= 16 ? m : m == 32 ? 8 : 16; }
+constexpr int row_plane_radix(int m) {
+    return m <= 16 ? m : m <= 64 ? 4 : m == 128 ? 8 : m == 256 ? 16 : 2;
+}
+// Twiddle table of those kernels: entry i is exp(-2 pi i k / n) with
+// k = regs_table_index(n, perThread, first, i).  Pass after pass, [r - 1][j]
+// with r < R, j < Ns and k = j r n / (Ns R); Ns is the product of the radices
+// before the pass.  The first radix is `first` (perThread when 0), the others
+// are perThread or what remains.
+constexpr int regs_table_size(int n, int perThread, int first = 0) {
+    const int ns = first > 0 ? first : perThread;
+    return n > ns ? n - ns : 1;
+}
+constexpr int regs_table_index(int n, int perThread, int first, int i) {
+    for (int ns = first > 0 ? first : perThread; ns < n;) {
+        const int radix = n / ns < perThread ? n / ns : perThread;
+        if (i < ns * (radix - 1)) return (i % ns) * (i / ns + 1) * (n / (ns * radix));
+        i -= ns * (radix - 1);
+        ns *= radix;
+    }
+    return 0;
+}
+// Where the entries of the pass with sub-transform size ns begin (radices
+// perThread, perThread, ... from the first).
+constexpr int regs_table_offset(int n, int perThread, int ns) {
+    (void)n;
+    return ns - perThread;
+}
+
 // x-direction transforms.  Planes [0, planes) of real volumes laid out
-// [plane][y][x]; bins kept for kx < keep.
+// [plane][y][x]; bins kept for kx < keep.  twHalf and the column transforms' tw
+// are tables in regs_table_index order: (Nx/2, row_regs_per_thread) forward,
+// the same with first radix row_plane_radix inverse, and (Ny,
+// column_regs_per_thread); twFull is the natural Nx-point table.
 cudaError_t launch_rows_forward(Precision p, int nx, int ny, long long planes, int keep, const void* real,
                                 DenseBins bins, const void* twHalf, const void* twFull, cudaStream_t stream);
 cudaError_t launch_rows_inverse(Precision p, int nx, int ny, long long planes, int keep, DenseBins bins, void* real,

@@ -83,25 +83,27 @@ std::size_t add_sat(std::size_t a, std::size_t b) {
 
 std::size_t round_up(std::size_t bytes) { return bytes > SIZE_MAX - 255 ? SIZE_MAX : (bytes + 255) & ~std::size_t(255); }
 
-// tw[k] = exp(-2 pi i k / n) for k in [0, n), the table layout the transform
-// kernels read.  sincospi of the exact dyadic argument 2k/n, rounded to T.
+// exp(-2 pi i k / n) at tw[i]: k = i for i in [0, n) (perThread 0), or the
+// regs_table_index order of the transform kernels, which has no more entries.
+// sincospi of the exact dyadic argument 2k/n, rounded to T.
 template <typename V>
-__global__ void fill_twiddles_kernel(V* tw, int n) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
+__global__ void fill_twiddles_kernel(V* tw, int n, int perThread, int first) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (perThread > 0 ? regs_table_size(n, perThread, first) : n)) return;
+    const int k = perThread > 0 ? regs_table_index(n, perThread, first, i) : i;
     double s, c;
     sincospi(2.0 * static_cast<double>(k) / static_cast<double>(n), &s, &c);
-    tw[k].x = static_cast<decltype(tw[k].x)>(c);
-    tw[k].y = static_cast<decltype(tw[k].y)>(-s);
+    tw[i].x = static_cast<decltype(tw[i].x)>(c);
+    tw[i].y = static_cast<decltype(tw[i].y)>(-s);
 }
 
-void fill_twiddles(Precision p, void* tw, int n, cudaStream_t s) {
+void fill_twiddles(Precision p, void* tw, int n, int perThread, int first, cudaStream_t s) {
     const int threads = 256;
     const int blocks = (n + threads - 1) / threads;
     if (p == Precision::f64)
-        fill_twiddles_kernel<<<blocks, threads, 0, s>>>(static_cast<double2*>(tw), n);
+        fill_twiddles_kernel<<<blocks, threads, 0, s>>>(static_cast<double2*>(tw), n, perThread, first);
     else
-        fill_twiddles_kernel<<<blocks, threads, 0, s>>>(static_cast<float2*>(tw), n);
+        fill_twiddles_kernel<<<blocks, threads, 0, s>>>(static_cast<float2*>(tw), n, perThread, first);
     check_cuda(cudaGetLastError(), "twiddle table kernel");
 }
 
@@ -140,9 +142,10 @@ void inverse_dense_static(const Workload& w, Precision p, const void* wvm, void*
     void* twCol = static_cast<unsigned char*>(twFull) + round_up(complexBytes * w.nx);
     void* bins = static_cast<unsigned char*>(twCol) + round_up(complexBytes * w.ny);
 
-    fill_twiddles(p, twHalf, half, s);
-    fill_twiddles(p, twFull, static_cast<int>(w.nx), s);
-    fill_twiddles(p, twCol, static_cast<int>(w.ny), s);
+    fill_twiddles(p, twHalf, half, row_regs_per_thread(half), row_plane_radix(half), s);
+    fill_twiddles(p, twFull, static_cast<int>(w.nx), 0, 0, s);
+    fill_twiddles(p, twCol, static_cast<int>(w.ny),
+                  column_regs_per_thread(static_cast<int>(w.ny), p == Precision::f64), 0, s);
     const int keep = static_cast<int>(w.nxHalf());
     const long long planes = static_cast<long long>(w.planes());
     const DenseBins in{const_cast<void*>(wvm), planes, keep};

@@ -47,6 +47,17 @@ int sm_count() {
 
 size_t element_bytes(Precision p) { return p == Precision::f64 ? sizeof(double) : sizeof(float); }
 
+std::vector<double> regs_table(const std::vector<double>& natural, int perThread, int first = 0) {
+    const int n = static_cast<int>(natural.size() / 2);
+    std::vector<double> out;
+    for (int i = 0; i < regs_table_size(n, perThread, first); ++i) {
+        const int k = regs_table_index(n, perThread, first, i);
+        out.push_back(natural[2 * k]);
+        out.push_back(natural[2 * k + 1]);
+    }
+    return out;
+}
+
 DeviceBuffer upload_real_table(const std::vector<double>& values, Precision p) {
     if (p == Precision::f64) return upload_vector(values);
     std::vector<float> f(values.begin(), values.end());
@@ -83,6 +94,11 @@ HorizontalPlan::HorizontalPlan(const Workload& w, Precision p, bool pruned, std:
     twHalf_ = upload_real_table(twHalf, p);
     twFull_ = upload_real_table(twFull, p);
     twCol_ = upload_real_table(twCol, p);
+    const int half = static_cast<int>(std::max<std::uint64_t>(1, w.nx / 2));
+    rowForward_ = upload_real_table(regs_table(twHalf, row_regs_per_thread(half)), p);
+    rowInverse_ = upload_real_table(regs_table(twHalf, row_regs_per_thread(half), row_plane_radix(half)), p);
+    colTable_ = upload_real_table(
+        regs_table(twCol, column_regs_per_thread(static_cast<int>(w.ny), p == Precision::f64)), p);
     cellMap_ = upload_vector(tables.cellMap);
     gatherMap_ = upload_vector(tables.gatherMap);
     colStart_ = upload_vector(tables.colStart);
@@ -91,7 +107,7 @@ HorizontalPlan::HorizontalPlan(const Workload& w, Precision p, bool pruned, std:
     modeKx_ = upload_vector(tables.modeKx);
     modeKy_ = upload_vector(tables.modeKy);
     modeConj_ = upload_vector(tables.modeConj);
-    const size_t binBytes = static_cast<size_t>(w.ny) * keep_ * maxPlanes * 2 * element_bytes(p);
+    const size_t binBytes = static_cast<size_t>(w.ny) * keep_ * (scratch_blocks(maxPlanes) << kScratchShift) * 2 * element_bytes(p);
     bins_.allocate(binBytes);
     {
         // Per-column band of the retained cells, and whether it is exact.
@@ -113,7 +129,7 @@ HorizontalPlan::HorizontalPlan(const Workload& w, Precision p, bool pruned, std:
         band_ = upload_vector(band);
     }
     allocationSeconds = seconds_since(allocStart);
-    persistentBytes = twHalf_.bytes() + twFull_.bytes() + twCol_.bytes() + cellMap_.bytes() + gatherMap_.bytes() +
+    persistentBytes = twHalf_.bytes() + twFull_.bytes() + twCol_.bytes() + rowForward_.bytes() + rowInverse_.bytes() + colTable_.bytes() + cellMap_.bytes() + gatherMap_.bytes() +
                       colStart_.bytes() +
                       colKy_.bytes() + colMode_.bytes() + modeKx_.bytes() + modeKy_.bytes() + modeConj_.bytes();
     scratchBytes = bins_.bytes();
@@ -126,7 +142,7 @@ ModeTables HorizontalPlan::tables() const {
 void HorizontalPlan::forward_rows(const void* real, std::uint64_t planes, cudaStream_t s) const {
     if (planes > maxPlanes_) throw Error(-1, "plane count exceeds the plan's scratch");
     check_cuda(launch_rows_forward(p_, static_cast<int>(w_.nx), static_cast<int>(w_.ny),
-                                   static_cast<long long>(planes), keep_, real, scratch(planes), twHalf_.get(),
+                                   static_cast<long long>(planes), keep_, real, scratch(planes), rowForward_.get(),
                                    twFull_.get(), s),
                "row r2c kernel");
 }
@@ -135,7 +151,7 @@ void HorizontalPlan::forward_columns(const ViewSet& views, double scale, cudaStr
     const auto planes = static_cast<std::uint64_t>(views.count) * w_.nz;
     if (planes > maxPlanes_) throw Error(-1, "plane count exceeds the plan's scratch");
     check_cuda(launch_columns_gather(p_, static_cast<int>(w_.ny), static_cast<int>(w_.nz), keep_, scratch(planes),
-                                     views, tables(), scale, twCol_.get(), s),
+                                     views, tables(), scale, colTable_.get(), s),
                "column c2c + retention kernel");
 }
 
@@ -143,7 +159,7 @@ void HorizontalPlan::inverse_columns(const ViewSet& views, cudaStream_t s) const
     const auto planes = static_cast<std::uint64_t>(views.count) * w_.nz;
     if (planes > maxPlanes_) throw Error(-1, "plane count exceeds the plan's scratch");
     check_cuda(launch_columns_embed(p_, static_cast<int>(w_.ny), static_cast<int>(w_.nz), keep_, views, tables(),
-                                    scratch(planes), twCol_.get(), s),
+                                    scratch(planes), colTable_.get(), s),
                "embedding + column c2c kernel");
 }
 
@@ -159,7 +175,7 @@ void HorizontalPlan::inverse_columns_into(const ViewSet& views, DenseBins out, c
     }
     if (zStride != nz) throw Error(-3, "padded bin planes need the FP32 warp column kernels");
     check_cuda(launch_columns_embed(p_, static_cast<int>(w_.ny), static_cast<int>(w_.nz), keep_, views, tables(), out,
-                                    twCol_.get(), s),
+                                    colTable_.get(), s),
                "embedding + column c2c kernel");
 }
 
@@ -176,7 +192,7 @@ void HorizontalPlan::forward_columns_from(DenseBins in, const ViewSet& views, do
     }
     if (zStride != nz) throw Error(-3, "padded bin planes need the FP32 warp column kernels");
     check_cuda(launch_columns_gather(p_, static_cast<int>(w_.ny), static_cast<int>(w_.nz), keep_, in, views,
-                                     tables(), scale, twCol_.get(), s),
+                                     tables(), scale, colTable_.get(), s),
                "column c2c + retention kernel");
 }
 
@@ -199,7 +215,7 @@ void HorizontalPlan::forward_columns_band(DenseBins bins, int slots, double scal
 void HorizontalPlan::inverse_rows(void* real, std::uint64_t planes, cudaStream_t s) const {
     if (planes > maxPlanes_) throw Error(-1, "plane count exceeds the plan's scratch");
     check_cuda(launch_rows_inverse(p_, static_cast<int>(w_.nx), static_cast<int>(w_.ny),
-                                   static_cast<long long>(planes), keep_, scratch(planes), real, twHalf_.get(),
+                                   static_cast<long long>(planes), keep_, scratch(planes), real, rowInverse_.get(),
                                    twFull_.get(), s),
                "row c2r kernel");
 }
@@ -221,10 +237,10 @@ void HorizontalPlan::forward_dense(const void* real, void* wvm, std::uint64_t pl
     if (keep_ != static_cast<int>(w_.nxHalf())) throw Error(-3, "dense transform requested from a pruned plan");
     const DenseBins out{wvm, static_cast<long long>(planes), static_cast<long long>(w_.nxHalf())};
     check_cuda(launch_rows_forward(p_, static_cast<int>(w_.nx), static_cast<int>(w_.ny),
-                                   static_cast<long long>(planes), keep_, real, out, twHalf_.get(), twFull_.get(), s),
+                                   static_cast<long long>(planes), keep_, real, out, rowForward_.get(), twFull_.get(), s),
                "row r2c kernel");
     check_cuda(launch_columns_dense(p_, -1, static_cast<int>(w_.ny), keep_, static_cast<long long>(planes), out, out,
-                                    twCol_.get(), s),
+                                    colTable_.get(), s),
                "column c2c kernel");
 }
 
@@ -233,10 +249,10 @@ void HorizontalPlan::inverse_dense(const void* wvm, void* real, std::uint64_t pl
     if (planes > maxPlanes_) throw Error(-1, "plane count exceeds the plan's scratch");
     const DenseBins in{const_cast<void*>(wvm), static_cast<long long>(planes), static_cast<long long>(w_.nxHalf())};
     check_cuda(launch_columns_dense(p_, +1, static_cast<int>(w_.ny), keep_, static_cast<long long>(planes), in,
-                                    scratch(planes), twCol_.get(), s),
+                                    scratch(planes), colTable_.get(), s),
                "column c2c kernel");
     check_cuda(launch_rows_inverse(p_, static_cast<int>(w_.nx), static_cast<int>(w_.ny),
-                                   static_cast<long long>(planes), keep_, scratch(planes), real, twHalf_.get(),
+                                   static_cast<long long>(planes), keep_, scratch(planes), real, rowInverse_.get(),
                                    twFull_.get(), s),
                "row c2r kernel");
 }

@@ -98,8 +98,14 @@ public:
     int keep() const { return keep_; }
     std::uint64_t modes() const { return modeCount_; }
     ModeTables tables() const;
-    DenseBins scratch(std::uint64_t planes) const {
-        return {bins_.get(), static_cast<long long>(planes), static_cast<long long>(keep_)};
+    // The scratch is plane-blocked.
+    std::uint64_t scratch_blocks(std::uint64_t planes) const {
+        return (planes + (std::uint64_t(1) << kScratchShift) - 1) >> kScratchShift;
+    }
+    DenseBins scratch(std::uint64_t) const {
+        const long long block = 1LL << kScratchShift;
+        return {bins_.get(), block, static_cast<long long>(keep_), kScratchShift,
+                block * static_cast<long long>(keep_) * static_cast<long long>(w_.ny)};
     }
 
     // x then y (forward) into views; y then x (inverse) from views.
@@ -147,9 +153,11 @@ private:
     std::uint64_t maxPlanes_ = 0;
     std::uint64_t modeCount_ = 0;
     DeviceBuffer twHalf_, twFull_, twCol_;
+    DeviceBuffer rowForward_, rowInverse_, colTable_;  // twHalf / twCol in regs_table_index order
     DeviceBuffer cellMap_, gatherMap_, colStart_, colKy_, colMode_, modeKx_, modeKy_, modeConj_;
     DeviceBuffer bins_;
     DeviceBuffer band_;
+    static constexpr int kScratchShift = 4;
     bool bandExact_ = false;
     int bandFormInverse_ = 0, bandFormForward_ = 0;
 };
