@@ -325,13 +325,6 @@ VerticalPlan::VerticalPlan(GemmPrecision p, int rowsOut, int inner, const std::v
         return;
     }
 
-    // SIMT forms read the transposed matrices At[g][s][r].
-    std::vector<double> At(groupsCount * matrixElems);
-    for (std::uint64_t g = 0; g < groupsCount; ++g)
-        for (int r = 0; r < rowsOut; ++r)
-            for (int s = 0; s < inner; ++s)
-                At[g * matrixElems + static_cast<std::uint64_t>(s) * rowsOut + r] =
-                    natural[g * matrixElems + static_cast<std::uint64_t>(r) * inner + s];
     const int width = gemm_tile_columns(p);
     std::vector<int> gc(groups.size()), gf(groups.size());
     for (std::uint64_t gi = 0; gi < groups.size(); ++gi) {
@@ -362,12 +355,31 @@ VerticalPlan::VerticalPlan(GemmPrecision p, int rowsOut, int inner, const std::v
         t.tiles = static_cast<int>(h.group.size());
         if (virtualTiles_) tilePrefix_[m - 1] = t.tiles;
     }
-    matrixStride_ = common ? 0 : static_cast<long long>(matrixElems);
     if (p == GemmPrecision::f64) {
-        matrices_ = upload_vector(At);
+        // Chunks of s, [chunk][r][s of the chunk] (vertical.hpp).
+        const int padded = gemm_f64_row(inner);
+        const std::uint64_t imageElems = static_cast<std::uint64_t>(rowsOut) * padded;
+        std::vector<double> images(groupsCount * imageElems, 0.0);
+        for (std::uint64_t g = 0; g < groupsCount; ++g)
+            for (int s0 = 0; s0 < inner; s0 += kGemmF64Chunk) {
+                const int chunk = gemm_f64_chunk_row(inner - s0);
+                double* to = images.data() + g * imageElems + static_cast<std::uint64_t>(s0) * rowsOut;
+                for (int r = 0; r < rowsOut; ++r)
+                    std::copy_n(natural.data() + g * matrixElems + static_cast<std::uint64_t>(r) * inner + s0,
+                                std::min(chunk, inner - s0), to + static_cast<std::uint64_t>(r) * chunk);
+            }
+        matrices_ = upload_vector(images);
+        matrixStride_ = common ? 0 : static_cast<long long>(imageElems);
     } else {
-        std::vector<float> f(At.begin(), At.end());
-        matrices_ = upload_vector(f);
+        // The FP32 form reads the transposed matrices At[g][s][r].
+        std::vector<float> At(groupsCount * matrixElems);
+        for (std::uint64_t g = 0; g < groupsCount; ++g)
+            for (int r = 0; r < rowsOut; ++r)
+                for (int s = 0; s < inner; ++s)
+                    At[g * matrixElems + static_cast<std::uint64_t>(s) * rowsOut + r] =
+                        static_cast<float>(natural[g * matrixElems + static_cast<std::uint64_t>(r) * inner + s]);
+        matrices_ = upload_vector(At);
+        matrixStride_ = common ? 0 : static_cast<long long>(matrixElems);
     }
     groupColumns_ = upload_vector(gc);
     groupFirst_ = upload_vector(gf);

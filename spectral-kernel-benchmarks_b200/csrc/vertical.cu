@@ -1,4 +1,4 @@
-// SIMT grouped vertical GEMM (FP64 / FP32).  See vertical.hpp.
+// SIMT grouped vertical GEMM (FP32; FP64 is vertical_f64.cu).  See vertical.hpp.
 //
 // One CTA of 256 threads computes a tile of 32 complex columns of one K^2
 // group, all R output rows.  The inner dimension S is streamed through shared
@@ -12,6 +12,7 @@
 #include "vertical.hpp"
 
 #include "fft_device.cuh"
+#include "vertical_device.cuh"
 
 namespace skb {
 namespace {
@@ -47,30 +48,6 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
-// Element offset of plan column `col` (member * memberColumns + mode * fields
-// + field) in a cell-addressed operand, with its partner (or -1) and
-// conjugation.
-__device__ __forceinline__ void bin_column(const BinBoundary& bb, int col, long long& base, long long& partner,
-                                           bool& conj) {
-    // Plan column = member * memberColumns + mode * fields + plan field.
-    long long member = 0;
-    int rest = col;
-    if (bb.memberColumns > 0) {
-        member = col / bb.memberColumns;
-        rest = static_cast<int>(col - member * bb.memberColumns);
-    }
-    const int mode = rest / bb.fields;
-    const int sub = rest - mode * bb.fields;
-    const int field = bb.fieldMap != nullptr ? __ldg(bb.fieldMap + sub) : sub;
-    const long long memberStride =
-        bb.memberStride != 0 ? bb.memberStride : static_cast<long long>(bb.fields) * bb.zStride;
-    const long long off = member * memberStride + static_cast<long long>(field) * bb.zStride;
-    base = __ldg(bb.cell + mode) + off;
-    const long long p = bb.partner != nullptr ? __ldg(bb.partner + mode) : -1;
-    partner = p >= 0 ? p + off : -1;
-    conj = bb.conj != nullptr && __ldg(bb.conj + mode) != 0;
 }
 
 template <typename T, int KR, bool SPLIT, bool BINS, bool VIRT>
@@ -279,7 +256,8 @@ cudaError_t launch_grouped_gemm(GemmPrecision p, int R, int S, const void* matri
     const BinBoundary ib = inBins ? *inBins : BinBoundary{};
     const BinBoundary ob = outBins ? *outBins : BinBoundary{};
     switch (p) {
-        case GemmPrecision::f64: return launch_t<double>(R, S, matrices, tiles, in, out, ib, ob, stream);
+        case GemmPrecision::f64:
+            return launch_grouped_gemm_f64(R, S, static_cast<const double*>(matrices), tiles, in, out, ib, ob, stream);
         case GemmPrecision::f32: return launch_t<float>(R, S, matrices, tiles, in, out, ib, ob, stream);
         default: return cudaErrorNotSupported;
     }

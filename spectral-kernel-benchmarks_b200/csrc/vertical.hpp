@@ -115,6 +115,20 @@ cudaError_t tc_gemm_build_images(const float* natural, int groups, int R, int S,
 int tc_gemm_unit_tiles();
 cudaError_t launch_tc_gemm(const TcGemmArgs& args, cudaStream_t stream);
 
+// FP64 form (vertical_f64.cu): matrices stored in chunks of kGemmF64Chunk along
+// s, [chunk][r][s of the chunk], zero-padded.  The last chunk has a multiple of
+// 4 values per row, and 4 more where that multiple is even (the shared copy's
+// bank pattern wants an odd one).
+constexpr int kGemmF64Chunk = 28;
+constexpr int gemm_f64_chunk_row(int left) { return left >= kGemmF64Chunk ? kGemmF64Chunk : (left + 3) / 4 * 4 | 4; }
+constexpr int gemm_f64_row(int S) {
+    const int full = S / kGemmF64Chunk * kGemmF64Chunk;
+    return full + (S > full ? gemm_f64_chunk_row(S - full) : 0);
+}
+cudaError_t launch_grouped_gemm_f64(int R, int S, const double* images, const GroupTiles& tiles, ComplexOperand in,
+                                    ComplexOperand out, const BinBoundary& inBins, const BinBoundary& outBins,
+                                    cudaStream_t stream);
+
 // inBins / outBins (optional): cell-addressed operands (BinBoundary) instead of
 // the compact [column][len] arrays.
 cudaError_t launch_grouped_gemm(GemmPrecision p, int R, int S, const void* matrices, const GroupTiles& tiles,
