@@ -86,7 +86,8 @@ __device__ __forceinline__ void dft_small(V* v) {
 }
 
 // One pass (sub-transforms of Ns points, radix R) on the thread's registers.
-template <typename S, int N, int E, int SIGN, int Ns>
+// LDG: the table lies in global memory (read through __ldg), else anywhere.
+template <typename S, int N, int E, int SIGN, int Ns, bool LDG = true>
 __device__ __forceinline__ void fft_regs_pass(cx<S> (&v)[E], int t, const cx<S>* tw) {
     using V = cx<S>;
     constexpr int T = N / E;
@@ -101,7 +102,8 @@ __device__ __forceinline__ void fft_regs_pass(cx<S> (&v)[E], int t, const cx<S>*
         if constexpr (Ns > 1) {
             const V* w = tw + (t + T * s) % Ns;
 #pragma unroll
-            for (int r = 1; r < R; ++r) b[r] = cmul(b[r], twiddle<SIGN>(w, Ns * (r - 1)));
+            for (int r = 1; r < R; ++r)
+                b[r] = cmul(b[r], LDG ? twiddle<SIGN>(w, Ns * (r - 1)) : twiddle_plain<SIGN>(w, Ns * (r - 1)));
         }
         dft_small<SIGN, R>(b);
 #pragma unroll
@@ -129,17 +131,17 @@ __device__ __forceinline__ void fft_regs_store(const cx<S> (&v)[E], int t, X& xc
 // of (at least) the T threads that share the sequence.  For Ns = 1 the exchange
 // buffer must be free on entry; loads of the last exchange may still be in
 // flight in other threads on return.
-template <typename S, int N, int E, int SIGN, int Ns = 1, typename X>
+template <typename S, int N, int E, int SIGN, int Ns = 1, bool LDG = true, typename X>
 __device__ __forceinline__ void fft_regs(cx<S> (&v)[E], int t, const cx<S>* tw, X& xch) {
     constexpr int R = N / Ns < E ? N / Ns : E;
-    fft_regs_pass<S, N, E, SIGN, Ns>(v, t, tw);
+    fft_regs_pass<S, N, E, SIGN, Ns, LDG>(v, t, tw);
     if constexpr (Ns * R < N) {
         if constexpr (Ns > 1) xch.fence();  // the previous exchange's loads
         fft_regs_store<S, N, E, Ns>(v, t, xch);
         xch.fence();
 #pragma unroll
         for (int e = 0; e < E; ++e) v[e] = xch.load(t + (N / E) * e);
-        fft_regs<S, N, E, SIGN, Ns * R>(v, t, Ns > 1 ? tw + Ns * (R - 1) : tw, xch);
+        fft_regs<S, N, E, SIGN, Ns * R, LDG>(v, t, Ns > 1 ? tw + Ns * (R - 1) : tw, xch);
     }
 }
 

@@ -271,28 +271,23 @@ __global__ void __launch_bounds__(32 * B, 16 / B) rows_flux_kernel(RowFluxArgs a
 // exchange per transform instead of two.  Lanes 0-15 own plane 2w of warp w,
 // lanes 16-31 plane 2w + 1.
 
-// 256-point FFT of one half-warp's sequence: v[m] = z[t + 16 m] in, Z[t + 16 k]
-// in v[k] out.  xch: this half-warp's 16 x 17 exchange region; tw2[16 k2 + t] =
-// exp(-2 pi i t k2 / 256) (conjugated for SIGN > 0).
-template <int SIGN>
-__device__ __forceinline__ void fft256_pair(float2 (&v)[16], float2* xch, const float2* tw2, int t) {
-    dft16<SIGN>(v);
-#pragma unroll
-    for (int k2 = 1; k2 < 16; ++k2) {
-        const float2 w = tw2[16 * k2 + t];
-        v[k2] = SIGN < 0 ? cmul(v[k2], w) : cmulc(v[k2], w);
-    }
-    __syncwarp();  // the previous transform's reads of xch are done
-#pragma unroll
-    for (int k2 = 0; k2 < 16; ++k2) xch[17 * t + k2] = v[k2];
-    __syncwarp();
-#pragma unroll
-    for (int n1 = 0; n1 < 16; ++n1) v[n1] = xch[17 * n1 + t];
-    dft16<SIGN>(v);
-}
+constexpr int kPairM = 256;  // half-length of the 512-point rows
+// Exchange words per plane: one spare per 16 makes the first pass's stride-16
+// stores conflict-free; for 128 and 64 points, whose access phases span two
+// and four planes, the region's length (8 and 4 mod 16) keeps those apart.
+constexpr int pair_xch(int M) { return M + M / 16; }
+// Bins the pre-processing reads: the 2/3 rule keeps kx < 11 T (T = M/16 lanes
+// per plane; 171 of 176, 86 of 88, 43 of 44), so bins k >= 11 T and, with them,
+// the products of registers m >= 11 (k) and m <= 4 (M - k) are left out.
+constexpr int pair_keep(int M) { return 11 * (M / 16); }
 
-constexpr int kPairM = 256;       // half-length of the 512-point rows
-constexpr int kPairXch = 16 * 17;  // exchange words per plane
+// A plane's exchange among its lanes.
+struct PairExchange {
+    float2* x;
+    __device__ __forceinline__ void store(int i, float2 v) { x[i + (i >> 4)] = v; }
+    __device__ __forceinline__ float2 load(int i) const { return x[i + (i >> 4)]; }
+    __device__ __forceinline__ void fence() const { __syncwarp(); }
+};
 template <int B>
 constexpr int pair_stage_row() {
     // kx = 0..M (the pre-processing reads X[M - k]), and a residue mod 16 (in
@@ -304,30 +299,30 @@ constexpr int pair_stage_row() {
 }
 template <int B>
 constexpr size_t pair_smem_words(int keep) {
-    return 2 * size_t(B) * pair_stage_row<B>() + size_t(B) * kPairXch + size_t(keep) * out_row<B>() + kPairM + kPairM;
+    return 2 * size_t(B) * pair_stage_row<B>() + size_t(B) * pair_xch(kPairM) + size_t(keep) * out_row<B>() + kPairM +
+           kPairM;
 }
 
-// TMA form of the stage: rows kx = 0..kTmaRows-1 (the pre-processing reads no
-// bin beyond kx = 176, see inverse_row), each row the B planes' values
+// TMA form of the stage: rows kx = 0..pair_keep(M) (the pre-processing reads
+// no bin beyond, see inverse_row), each row the B planes' values
 // (64 or 128 bytes) in the SWIZZLE_64B / SWIZZLE_128B pattern the tensor
-// copy writes; rows keep..kTmaRows-1 are zero.  Stages start on 1024-byte
+// copy writes; rows keep..pair_keep(M) are zero.  Stages start on 1024-byte
 // boundaries (the swizzle pattern's period).
-constexpr int kTmaRows = 177;
-template <int B>
+template <int M, int B>
 constexpr size_t tma_stage_bytes() {
-    return (size_t(kTmaRows) * B * 8 + 1023) / 1024 * 1024;
+    return (size_t(pair_keep(M) + 1) * B * 8 + 1023) / 1024 * 1024;
 }
-// W_SMEM: the third velocity row W is kept in a lane-private shared region
-// (16 values per thread) instead of registers.
-template <int B, int MINB, int NS>
+// The third velocity row W is kept in a lane-private shared region (16 values
+// per thread) instead of registers in the forms compiled for 12 warps per SM.
+template <int M, int B, int MINB, int NS>
 constexpr bool pair_w_in_smem() {
-    return B == 8 && MINB == 3 && NS == 2;
+    return NS == 2 && MINB * M * B == 3 * 256 * 8;
 }
-template <int B, int NS, bool WSM = false>
+template <int M, int B, int NS, bool WSM>
 constexpr size_t pair_tma_smem_bytes(int keep) {
-    return 1024 + NS * tma_stage_bytes<B>() +
-           sizeof(float2) * (size_t(B) * kPairXch + size_t(keep) * out_row<B>() + kPairM + kPairM +
-                             (WSM ? size_t(16) * 16 * B : 0));
+    return 1024 + NS * tma_stage_bytes<M, B>() +
+           sizeof(float2) * (size_t(B) * pair_xch(M) + size_t(keep) * out_row<B>() + M + M +
+                             (WSM ? size_t(M) * B : 0));
 }
 // Byte offset of (kx k, plane b) in a swizzled TMA stage.
 template <int B>
@@ -364,15 +359,16 @@ __device__ __forceinline__ bool stage_wait(unsigned bar, unsigned parity, long l
 // ahead of the one being transformed.  Thread 0's bounded wait on the copy is
 // folded into the slot's CTA barrier (__syncthreads_and), so an expired wait
 // makes every thread leave together after setting the error word.
-template <int B, int MINB, int NS>
-__global__ void __launch_bounds__(16 * B, MINB)
+template <int M, int B, int MINB, int NS>
+__global__ void __launch_bounds__(M / 16 * B, MINB)
     rows_flux_pair_kernel(RowFluxArgs a, const __grid_constant__ CUtensorMap tmIn) {
     using V = float2;
     constexpr bool TMA = NS != 0;
     constexpr int NST = TMA ? NS : 2;  // stages
-    constexpr int M = kPairM;
-    constexpr int NT = 16 * B;
+    constexpr int T = M / 16;  // lanes per plane
+    constexpr int NT = T * B;
     constexpr int KP = pair_stage_row<B>();
+    static_assert(M == kPairM || TMA, "the cp.async stages are laid out for 512-point rows");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ __align__(8) unsigned long long stageFull[NST];
     __shared__ __align__(8) unsigned long long never;  // nothing arrives on it (expired-wait test)
@@ -381,24 +377,24 @@ __global__ void __launch_bounds__(16 * B, MINB)
         reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     auto stage_of = [&](int f) -> V* {
         if constexpr (TMA)
-            return reinterpret_cast<V*>(tmaBase + (f % NST) * tma_stage_bytes<B>());
+            return reinterpret_cast<V*>(tmaBase + (f % NST) * tma_stage_bytes<M, B>());
         else
             return reinterpret_cast<V*>(smem_raw) + (f & 1) * B * KP;
     };
     V* stage0 = stage_of(0);
-    V* xchAll = TMA ? reinterpret_cast<V*>(tmaBase + NST * tma_stage_bytes<B>()) : stage0 + 2 * B * KP;
-    V* outTile = xchAll + B * kPairXch;  // [k][b] at out_slot(k, b)
+    V* xchAll = TMA ? reinterpret_cast<V*>(tmaBase + NST * tma_stage_bytes<M, B>()) : stage0 + 2 * B * KP;
+    V* outTile = xchAll + B * pair_xch(M);  // [k][b] at out_slot(k, b)
     V* tf = outTile + keep * out_row<B>();  // twFull[0..M)
-    V* tw2 = tf + M;                     // tw2[16 k2 + t] = twHalf[(t k2) mod M]
-    // Three-CTA two-stage TMA form: W (16 values per thread) lives here, at
-    // wsm[16 * e ... ] + tid, which takes the register peak of u, v, w, the
+    V* tw2 = tf + M;                     // fft_regs' table: tw2[16 (r - 1) + j] = twHalf[j r]
+    // Two-stage TMA forms at 12 warps per SM: W (16 values per thread) lives
+    // here, at wsm[e * NT + tid], which takes the register peak of u, v, w, the
     // product and the current derivative under the 168-register bound.
-    constexpr bool WSM = pair_w_in_smem<B, MINB, NS>();
+    constexpr bool WSM = pair_w_in_smem<M, B, MINB, NS>();
     V* wsm = tw2 + M;
     const int tid = threadIdx.x;
-    const int warp = tid >> 5, lane = tid & 31;
-    const int t = lane & 15;
-    const int pl = 2 * warp + (lane >> 4);  // this half-warp's plane within the CTA
+    const int lane = tid & 31;
+    const int t = tid % T;
+    const int pl = tid / T;  // these lanes' plane within the CTA
     const int zChunks = (a.nz + B - 1) / B;
     const int member = blockIdx.x / zChunks;
     const int z0 = (blockIdx.x % zChunks) * B;
@@ -409,19 +405,19 @@ __global__ void __launch_bounds__(16 * B, MINB)
     V* out = static_cast<V*>(a.binsOut.data);
     const long long inRow = a.binsIn.planes;
     const long long outRow = a.binsOut.planes;
-    V* xch = xchAll + pl * kPairXch;
+    PairExchange xch{xchAll + pl * pair_xch(M)};
 
     for (int i = tid; i < M; i += NT) {
         tf[i] = twFull[i];
-        tw2[i] = twHalf[((i & 15) * (i >> 4)) & (M - 1)];
+        if (i < M - 16) tw2[i] = twHalf[(i & 15) * ((i >> 4) + 1)];
     }
     if constexpr (TMA) {
-        // Rows keep..kTmaRows-1 of every stage are zero (the tensor copies
+        // Rows keep..pair_keep(M) of every stage are zero (the tensor copies
         // write rows 0..keep-1 only; the swizzle stays inside a row).
-        for (int i = tid; i < NST * (kTmaRows - keep) * B; i += NT) {
-            const int st = i / ((kTmaRows - keep) * B);
-            const int j = i % ((kTmaRows - keep) * B);
-            reinterpret_cast<V*>(tmaBase + st * tma_stage_bytes<B>())[keep * B + j] = V{0.f, 0.f};
+        const int zeros = (pair_keep(M) + 1 - keep) * B;
+        for (int i = tid; i < NST * zeros; i += NT) {
+            const int st = i / zeros;
+            reinterpret_cast<V*>(tmaBase + st * tma_stage_bytes<M, B>())[keep * B + i - st * zeros] = V{0.f, 0.f};
         }
         if (tid == 0) {
             for (int i = 0; i < NST; ++i)
@@ -445,8 +441,15 @@ __global__ void __launch_bounds__(16 * B, MINB)
     const int cb = tid % B;
     const int ck = tid / B;
     const bool cok = z0 + cb < a.nz;
-    const int tmaLo = static_cast<int>(tma_stage_offset<B>(t, pl));
-    const int tmaHi = static_cast<int>(tma_stage_offset<B>(M - t, pl));
+    // This lane's byte offsets of bins t and M - t; the swizzle repeats every 8
+    // rows, so with fewer than 8 lanes per plane register m = 1 has its own.
+    constexpr int PER = T < 8 ? 8 / T : 1;
+    int tmaLo[PER], tmaHi[PER];
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        tmaLo[i] = static_cast<int>(tma_stage_offset<B>(t + T * i, pl));
+        tmaHi[i] = static_cast<int>(tma_stage_offset<B>(M - t - T * i, pl));
+    }
     auto issue = [&](int f) {
         V* stage = stage_of(f);
         if constexpr (TMA) {
@@ -497,21 +500,22 @@ __global__ void __launch_bounds__(16 * B, MINB)
         if (f + NST - 1 < a.fieldsIn) issue(f + NST - 1);
         const V* st = stage_of(f) + pl * KP;
         const unsigned char* stb = reinterpret_cast<const unsigned char*>(stage_of(f));
-        // TMA form: bins k = t + 16 m and M - k sit at this lane's swizzled
-        // offsets of m = 0 plus or minus m rows of 16 (16 * B * 8 bytes, a
-        // multiple of the swizzle period, so the pattern repeats).
+        // TMA form: bins k = t + T m and M - k sit at this lane's swizzled
+        // offsets plus or minus whole swizzle periods.
         auto bin = [&](int m, bool mirror) -> V {
-            if constexpr (TMA)
-                return *reinterpret_cast<const V*>(stb + (mirror ? tmaHi - m * 128 * B : tmaLo + m * 128 * B));
-            else
-                return st[mirror ? M - t - 16 * m : t + 16 * m];
+            if constexpr (TMA) {
+                const int rows = (m / PER) * PER * T * B * 8;
+                return *reinterpret_cast<const V*>(stb + (mirror ? tmaHi[m % PER] - rows : tmaLo[m % PER] + rows));
+            } else {
+                return st[mirror ? M - t - T * m : t + T * m];
+            }
         };
-        // keep <= 176 (checked at launch): bins k >= 176 (m >= 11) and
-        // M - k >= 177 (m <= 4) lie beyond the 2/3 band and are zero, so those
+        // keep <= 11 T (checked at launch): bins k >= 11 T (m >= 11) and
+        // M - k > 11 T (m <= 4) lie beyond the 2/3 band and are zero, so those
         // shared-memory reads are left out.
 #pragma unroll
         for (int m = 0; m < 16; ++m) {
-            const int k = t + 16 * m;
+            const int k = t + T * m;
             V xk = m < 11 ? bin(m, false) : V{0.f, 0.f};
             V xm = m > 4 ? bin(m, true) : V{0.f, 0.f};
             if (m == 0 && t == 0) {  // bins 0 and M are real
@@ -523,7 +527,8 @@ __global__ void __launch_bounds__(16 * B, MINB)
             const V tt = cmulc(d, tf[k]);
             r[m] = {sum.x - tt.y, sum.y + tt.x};
         }
-        fft256_pair<+1>(r, xch, tw2, t);
+        __syncwarp();  // the previous transform's reads of the exchange are done
+        fft_regs<float, M, 16, +1, 1, false>(r, t, tw2, xch);
         return true;
     };
 
@@ -536,7 +541,7 @@ __global__ void __launch_bounds__(16 * B, MINB)
         for (int e = 0; e < 16; ++e) wsm[e * NT + tid] = w[e];
     }
     const float scale = a.scale;
-    const int src = ((16 - t) & 15) + (lane & 16);  // lane holding Z[M - k]
+    const int src = ((T - t) & (T - 1)) + (lane & ~(T - 1));  // lane holding Z[M - k]
     for (int tg = 0; tg < a.targets; ++tg) {
         V acc[16], q[16];
         if (!inverse_row(3 + 3 * tg, q)) return;
@@ -551,15 +556,16 @@ __global__ void __launch_bounds__(16 * B, MINB)
             const V we = WSM ? wsm[e * NT + tid] : w[e];
             acc[e] = {-scale * (acc[e].x + we.x * q[e].x), -scale * (acc[e].y + we.y * q[e].y)};
         }
-        fft256_pair<-1>(acc, xch, tw2, t);
-        // Real-spectrum split, kx < keep, into [k][b].  Z[M - k] for k = t + 16 k1
-        // is register 15 - k1 of lane 16 - t (t > 0) or register (16 - k1) mod 16
+        __syncwarp();
+        fft_regs<float, M, 16, -1, 1, false>(acc, t, tw2, xch);
+        // Real-spectrum split, kx < keep, into [k][b].  Z[M - k] for k = t + T k1
+        // is register 15 - k1 of lane T - t (t > 0) or register (16 - k1) mod 16
         // of this lane (t = 0).
 #pragma unroll
-        for (int k1 = 0; k1 < 11; ++k1) {  // k < 176 >= keep
+        for (int k1 = 0; k1 < 11; ++k1) {  // k < 11 T >= keep
             const V other = {__shfl_sync(0xFFFFFFFFu, acc[15 - k1].x, src),
                              __shfl_sync(0xFFFFFFFFu, acc[15 - k1].y, src)};
-            const int k = t + 16 * k1;
+            const int k = t + T * k1;
             const V zk = acc[k1];
             const V zm = cconj(t == 0 ? acc[(16 - k1) & 15] : other);
             V X;
@@ -583,12 +589,12 @@ __global__ void __launch_bounds__(16 * B, MINB)
     }
 }
 
-template <int B, int MINB, int NS>
+template <int M, int B, int MINB, int NS>
 cudaError_t launch_pair(const RowFluxArgs& a, cudaStream_t stream) {
     constexpr bool TMA = NS != 0;
     const int zChunks = (a.nz + B - 1) / B;
     const dim3 grid(unsigned(zChunks * a.members), unsigned(a.ny));
-    auto kernel = rows_flux_pair_kernel<B, MINB, NS>;
+    auto kernel = rows_flux_pair_kernel<M, B, MINB, NS>;
     CUtensorMap map{};
     size_t bytes = sizeof(float2) * pair_smem_words<B>(a.keep);
     if constexpr (TMA) {
@@ -599,22 +605,31 @@ cudaError_t launch_pair(const RowFluxArgs& a, cudaStream_t stream) {
                                   static_cast<unsigned long long>(a.ny) * a.binsIn.kxStride,
                                   static_cast<unsigned long long>(a.binsIn.planes) * 8, B, a.keep);
         if (merr != cudaSuccess) return merr;
-        bytes = pair_tma_smem_bytes<B, NS, pair_w_in_smem<B, MINB, NS>()>(a.keep);
+        bytes = pair_tma_smem_bytes<M, B, NS, pair_w_in_smem<M, B, MINB, NS>()>(a.keep);
     }
     const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
     if (err != cudaSuccess) return err;
-    kernel<<<grid, 16 * B, bytes, stream>>>(a, map);
+    kernel<<<grid, M / 16 * B, bytes, stream>>>(a, map);
     return cudaGetLastError();
 }
 
 template <int NS>
 cudaError_t launch_pair_form(const RowFluxArgs& a, cudaStream_t stream) {
-    if (a.planes == 8) return a.pairs == 2 ? launch_pair<8, 3, NS>(a, stream) : launch_pair<8, 2, NS>(a, stream);
-    if (a.planes == 16) return launch_pair<16, 1, NS>(a, stream);
+    constexpr int M = kPairM;
+    if (a.planes == 8) return a.pairs == 2 ? launch_pair<M, 8, 3, NS>(a, stream) : launch_pair<M, 8, 2, NS>(a, stream);
+    if (a.planes == 16) return launch_pair<M, 16, 1, NS>(a, stream);
     // 24 planes (12 warps, one CTA per SM, 192-byte pieces): cp.async only,
     // no TMA swizzle pattern fits a 192-byte row.
-    if (a.planes == 24) return launch_pair<24, 1, 0>(a, stream);
+    if (a.planes == 24) return launch_pair<M, 24, 1, 0>(a, stream);
     return cudaErrorInvalidValue;
+}
+
+// 256- and 128-point rows: four or eight planes per warp, TMA stages, at the
+// same 12 warps per SM.
+template <int M>
+cudaError_t launch_short_rows(const RowFluxArgs& a, cudaStream_t stream) {
+    if (a.planes >= 16) return launch_pair<M, 16, 3 * 256 * 8 / (M * 16), 2>(a, stream);
+    return launch_pair<M, 8, 3 * 256 * 8 / (M * 8), 2>(a, stream);
 }
 
 }  // namespace
@@ -646,17 +661,19 @@ cudaError_t launch_planes(const RowFluxArgs& a, cudaStream_t stream) {
 cudaError_t launch_rows_flux(const RowFluxArgs& a, cudaStream_t stream) {
     const int M = a.nx / 2;
     if (a.keep < 1 || a.keep > M + 1 || a.fieldsIn != 3 + 3 * a.targets || a.zStride < a.nz) return cudaErrorInvalidValue;
-    if (a.pairs != 0 && M == kPairM && a.keep <= 176 && (a.planes == 8 || a.planes == 16 || a.planes == 24)) {
-        // The TMA form needs the error word (its copy waits are bounded) and
-        // 16-byte aligned cells.
-        const bool tma = a.tma != 0 && a.error != nullptr && a.binsIn.planes % 2 == 0 && a.zStride % 2 == 0;
-        if (!tma) return launch_pair_form<0>(a, stream);
+    // The TMA forms need the error word (their copy waits are bounded) and
+    // 16-byte aligned cells.
+    const bool tmaReady = a.error != nullptr && a.binsIn.planes % 2 == 0 && a.zStride % 2 == 0;
+    if (M == 128 || M == 64) {
+        if (!tmaReady || a.keep > pair_keep(M)) return cudaErrorInvalidValue;
+        return M == 128 ? launch_short_rows<128>(a, stream) : launch_short_rows<64>(a, stream);
+    }
+    if (a.pairs != 0 && M == kPairM && a.keep <= pair_keep(M) && (a.planes == 8 || a.planes == 16 || a.planes == 24)) {
+        if (a.tma == 0 || !tmaReady) return launch_pair_form<0>(a, stream);
         return a.tma == 2 ? launch_pair_form<3>(a, stream) : launch_pair_form<2>(a, stream);
     }
     switch (M) {
         case 32: return launch_planes<32>(a, stream);
-        case 64: return launch_planes<64>(a, stream);
-        case 128: return launch_planes<128>(a, stream);
         case 256: return launch_planes<256>(a, stream);
         default: return cudaErrorInvalidValue;
     }
