@@ -15,7 +15,7 @@
 
 #include <algorithm>
 #include "async_copy.cuh"
-#include "fft_device.cuh"
+#include "fft_regs.cuh"
 
 namespace skb {
 namespace {
@@ -586,7 +586,63 @@ __global__ void __launch_bounds__(256, 2) columns_band_persist_kernel(int nz, in
     }
 }
 
-// Generic-N band forms (warp per plane, cp.async staging).
+// Band columns of up to 256 points (and a 512-point form), register-ended
+// (fft_regs.cuh): 16 planes of the flat plane index (slot * zStride + z) and one
+// kx column per CTA; thread (plane b, t) loads its N/T elements from HBM into
+// registers and stores them back, with one shared exchange between (two at 512
+// points) where the warp-per-plane form staged loads, passes and results
+// through shared memory (84 % of the L1 pipe, 32 % of HBM).  Planes of the slot
+// padding (z >= Nz) are skipped.  Bound: load latency at 28 warps per SM, then
+// HBM (54 %).  256 points, 48 slots of 65 planes (835 MB): inverse 320 -> 205 us,
+// forward (12 slots) 81 -> 51 us; 128 points, 12 slots of 33: 19 -> 12 us.  At 512
+// points (15 slots of 129) 559 us against 532 of the pipelined form, forward (4
+// slots) 138 us against 146 of the next best: a tuner candidate.
+template <int N>
+struct BandRegs {
+    static constexpr int B = 16;
+    static constexpr int E = column_regs_per_thread(N, false);
+    static constexpr int T = N / E;
+    static constexpr int NT = B * T;
+    static constexpr int kCtas = 65536 / (NT * (E > 8 ? 64 : 40)) > 16 ? 16 : 65536 / (NT * (E > 8 ? 64 : 40));
+    static constexpr size_t kBytes = sizeof(float2) * N * B;
+};
+
+template <int N, int SIGN>
+__global__ void __launch_bounds__(BandRegs<N>::NT, BandRegs<N>::kCtas)
+    columns_band_regs_kernel(int nz, int zStride, long long planes, DenseBins bins, const int* __restrict__ bandOf,
+                             float scale, const float2* __restrict__ table) {
+    using C = BandRegs<N>;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int b = threadIdx.x % C::B;
+    const int t = threadIdx.x / C::B;
+    const long long p = (long long)blockIdx.x * C::B + b;
+    const int kx = blockIdx.y;
+    const int band = __ldg(bandOf + kx);
+    const bool live = p < planes && static_cast<int>(p % zStride) < nz;
+    const long long rowStride = bins.planes * bins.kxStride;
+    float2* const col = static_cast<float2*>(bins.data) + (live ? p : 0) + bins.planes * kx + rowStride * t;
+    const long long step = rowStride * C::T;
+    float2 v[C::E];
+    const float2* from = col;
+#pragma unroll
+    for (int e = 0; e < C::E; ++e, from += step) {
+        const bool have = live && (SIGN < 0 || in_band(t + C::T * e, N, band));
+        v[e] = have ? *from : make_float2(0.f, 0.f);
+    }
+    PlaneExchange<float2, C::B> xch{reinterpret_cast<float2*>(smem_raw) + b};
+    fft_regs<float, N, C::E, SIGN>(v, t, table, xch);
+    if (!live) return;
+    float2* to = col;
+#pragma unroll
+    for (int e = 0; e < C::E; ++e, to += step) {
+        if (SIGN > 0)
+            *to = v[e];
+        else if (in_band(t + C::T * e, N, band))
+            *to = make_float2(scale * v[e].x, scale * v[e].y);
+    }
+}
+
+// 512-point band forms with a warp per plane and cp.async staging.
 template <int N, int B>
 __global__ void __launch_bounds__(32 * B, 4) columns_inverse_band_warp_kernel(int nz, int zStride, DenseBins bins,
                                                                               const int* __restrict__ bandOf,
@@ -931,28 +987,42 @@ cudaError_t launch_band_persist(int nz, int zStride, int slots, int columns, Den
     return cudaGetLastError();
 }
 
-template <int N>
-cudaError_t inverse_band_n(int nz, int zStride, int slots, int columns, DenseBins bins, const int* band, const void* tw,
-                           int form, cudaStream_t s) {
+template <int N, int SIGN>
+cudaError_t launch_band_regs(int nz, int zStride, int slots, int columns, DenseBins bins, const int* band, float scale,
+                             const void* table, cudaStream_t s) {
+    using C = BandRegs<N>;
+    auto kernel = columns_band_regs_kernel<N, SIGN>;
+    const cudaError_t err = prepare(kernel, C::kBytes);
+    if (err != cudaSuccess) return err;
+    const long long planes = static_cast<long long>(slots) * zStride;
+    const dim3 grid(unsigned((planes + C::B - 1) / C::B), unsigned(columns));
+    kernel<<<grid, C::NT, C::kBytes, s>>>(nz, zStride, planes, bins, band, scale, static_cast<const float2*>(table));
+    return cudaGetLastError();
+}
+
+cudaError_t inverse_band_512(int nz, int zStride, int slots, int columns, DenseBins bins, const int* band, const void* tw,
+                             const void* table, int form, cudaStream_t s) {
     constexpr int B = 8;
     const int zChunks = (nz + B - 1) / B;
+    if (form == kBandRegs)
+        return launch_band_regs<kDirectN, +1>(nz, zStride, slots, columns, bins, band, 1.0f, table, s);
     const dim3 grid(unsigned(zChunks * slots), unsigned(columns));
-    if (N == kDirectN && form == kBandPersist)
+    if (form == kBandPersist)
         return launch_band_persist<+1>(nz, zStride, slots, columns, bins, band, 1.0f, tw, s);
-    if (N == kDirectN && form == kBand16)
+    if (form == kBand16)
         return launch_band_wide<16, +1>(nz, zStride, slots, columns, bins, band, 1.0f, tw, s);
-    if (N == kDirectN && form == kBand32)
+    if (form == kBand32)
         return launch_band_wide<32, +1>(nz, zStride, slots, columns, bins, band, 1.0f, tw, s);
-    if (N == kDirectN && band_pipe_columns(form) > 0)
+    if (band_pipe_columns(form) > 0)
         return launch_band_pipe<+1>(nz, zStride, slots, columns, bins, band, 1.0f, tw, band_pipe_columns(form), s);
-    if (N == kDirectN && form != kBandWarp) {
+    if (form != kBandWarp) {
         auto kernel = form == kBandDirect4 ? columns_inverse_band_kernel<4> : columns_inverse_band_kernel<3>;
         cudaError_t err = prepare(kernel, kDirectSmem);
         if (err != cudaSuccess) return err;
         kernel<<<grid, 256, kDirectSmem, s>>>(nz, zStride, bins, band, static_cast<const float2*>(tw));
     } else {
-        auto kernel = columns_inverse_band_warp_kernel<N, B>;
-        const size_t bytes = sizeof(float2) * size_t(B) * plane_region<N>();
+        auto kernel = columns_inverse_band_warp_kernel<kDirectN, B>;
+        const size_t bytes = sizeof(float2) * size_t(B) * plane_region<kDirectN>();
         cudaError_t err = prepare(kernel, bytes);
         if (err != cudaSuccess) return err;
         kernel<<<grid, 32 * B, bytes, s>>>(nz, zStride, bins, band, static_cast<const float2*>(tw));
@@ -960,28 +1030,29 @@ cudaError_t inverse_band_n(int nz, int zStride, int slots, int columns, DenseBin
     return cudaGetLastError();
 }
 
-template <int N>
-cudaError_t forward_band_n(int nz, int zStride, int slots, int columns, DenseBins bins, const int* band, double scale,
-                           const void* tw, int form, cudaStream_t s) {
+cudaError_t forward_band_512(int nz, int zStride, int slots, int columns, DenseBins bins, const int* band, double scale, const void* tw,
+                             const void* table, int form, cudaStream_t s) {
     constexpr int B = 8;
     const int zChunks = (nz + B - 1) / B;
+    if (form == kBandRegs)
+        return launch_band_regs<kDirectN, -1>(nz, zStride, slots, columns, bins, band, float(scale), table, s);
     const dim3 grid(unsigned(zChunks * slots), unsigned(columns));
-    if (N == kDirectN && form == kBandPersist)
+    if (form == kBandPersist)
         return launch_band_persist<-1>(nz, zStride, slots, columns, bins, band, float(scale), tw, s);
-    if (N == kDirectN && form == kBand16)
+    if (form == kBand16)
         return launch_band_wide<16, -1>(nz, zStride, slots, columns, bins, band, float(scale), tw, s);
-    if (N == kDirectN && form == kBand32)
+    if (form == kBand32)
         return launch_band_wide<32, -1>(nz, zStride, slots, columns, bins, band, float(scale), tw, s);
-    if (N == kDirectN && band_pipe_columns(form) > 0)
+    if (band_pipe_columns(form) > 0)
         return launch_band_pipe<-1>(nz, zStride, slots, columns, bins, band, float(scale), tw, band_pipe_columns(form), s);
-    if (N == kDirectN && form != kBandWarp) {
+    if (form != kBandWarp) {
         auto kernel = form == kBandDirect4 ? columns_forward_band_kernel<4> : columns_forward_band_kernel<3>;
         cudaError_t err = prepare(kernel, kDirectSmem);
         if (err != cudaSuccess) return err;
         kernel<<<grid, 256, kDirectSmem, s>>>(nz, zStride, bins, band, float(scale), static_cast<const float2*>(tw));
     } else {
-        auto kernel = columns_forward_band_warp_kernel<N, B>;
-        const size_t bytes = sizeof(float2) * size_t(B) * plane_region<N>();
+        auto kernel = columns_forward_band_warp_kernel<kDirectN, B>;
+        const size_t bytes = sizeof(float2) * size_t(B) * plane_region<kDirectN>();
         cudaError_t err = prepare(kernel, bytes);
         if (err != cudaSuccess) return err;
         kernel<<<grid, 32 * B, bytes, s>>>(nz, zStride, bins, band, float(scale), static_cast<const float2*>(tw));
@@ -1038,27 +1109,28 @@ cudaError_t launch_columns_gather_warp(int ny, int nz, int zStride, int columns,
 namespace skb {
 
 cudaError_t launch_columns_inverse_band(int ny, int nz, int zStride, int slots, int columns, DenseBins bins,
-                                        const int* band, const void* tw, int form, cudaStream_t s) {
+                                        const int* band, const void* tw, const void* table, int form, cudaStream_t s) {
     if (slots <= 0 || columns <= 0) return cudaSuccess;
     switch (ny) {
-        case 32: return inverse_band_n<32>(nz, zStride, slots, columns, bins, band, tw, form, s);
-        case 64: return inverse_band_n<64>(nz, zStride, slots, columns, bins, band, tw, form, s);
-        case 128: return inverse_band_n<128>(nz, zStride, slots, columns, bins, band, tw, form, s);
-        case 256: return inverse_band_n<256>(nz, zStride, slots, columns, bins, band, tw, form, s);
-        case 512: return inverse_band_n<512>(nz, zStride, slots, columns, bins, band, tw, form, s);
+        case 32: return launch_band_regs<32, +1>(nz, zStride, slots, columns, bins, band, 1.0f, table, s);
+        case 64: return launch_band_regs<64, +1>(nz, zStride, slots, columns, bins, band, 1.0f, table, s);
+        case 128: return launch_band_regs<128, +1>(nz, zStride, slots, columns, bins, band, 1.0f, table, s);
+        case 256: return launch_band_regs<256, +1>(nz, zStride, slots, columns, bins, band, 1.0f, table, s);
+        case 512: return inverse_band_512(nz, zStride, slots, columns, bins, band, tw, table, form, s);
         default: return cudaErrorInvalidValue;
     }
 }
 
 cudaError_t launch_columns_forward_band(int ny, int nz, int zStride, int slots, int columns, DenseBins bins,
-                                        const int* band, double scale, const void* tw, int form, cudaStream_t s) {
+                                        const int* band, double scale, const void* tw, const void* table, int form,
+                                        cudaStream_t s) {
     if (slots <= 0 || columns <= 0) return cudaSuccess;
     switch (ny) {
-        case 32: return forward_band_n<32>(nz, zStride, slots, columns, bins, band, scale, tw, form, s);
-        case 64: return forward_band_n<64>(nz, zStride, slots, columns, bins, band, scale, tw, form, s);
-        case 128: return forward_band_n<128>(nz, zStride, slots, columns, bins, band, scale, tw, form, s);
-        case 256: return forward_band_n<256>(nz, zStride, slots, columns, bins, band, scale, tw, form, s);
-        case 512: return forward_band_n<512>(nz, zStride, slots, columns, bins, band, scale, tw, form, s);
+        case 32: return launch_band_regs<32, -1>(nz, zStride, slots, columns, bins, band, float(scale), table, s);
+        case 64: return launch_band_regs<64, -1>(nz, zStride, slots, columns, bins, band, float(scale), table, s);
+        case 128: return launch_band_regs<128, -1>(nz, zStride, slots, columns, bins, band, float(scale), table, s);
+        case 256: return launch_band_regs<256, -1>(nz, zStride, slots, columns, bins, band, float(scale), table, s);
+        case 512: return forward_band_512(nz, zStride, slots, columns, bins, band, scale, tw, table, form, s);
         default: return cudaErrorInvalidValue;
     }
 }

@@ -22,10 +22,10 @@ cudaError_t launch_columns_gather_warp(int ny, int nz, int zStride, int columns,
 // f: f * zStride + z): band[kx] bounds the retained cells of column kx
 // (min(ky, Ny - ky) <= band[kx]).  Inverse: band cells in, whole column out.
 // Forward: whole column in, band cells (times scale) out.
-// Band kernel forms: kBandDefault is the direct three-pass kernel at Ny = 512
-// and the warp-per-plane kernel below; kBandWarp selects the warp-per-plane
-// kernel at every size; kBandPersist the persistent direct kernel (Ny = 512
-// only), which loads the next tile during the current one's passes;
+// Up to Ny = 256 one register-ended kernel serves (16 planes per CTA); the forms
+// are those of Ny = 512: kBandDefault is the direct three-pass kernel; kBandWarp
+// the warp-per-plane kernel; kBandPersist the persistent direct kernel, which
+// loads the next tile during the current one's passes;
 // kBandDirect4 the direct kernel compiled for four resident CTAs per SM
 // instead of three (at most 64 registers a thread), for more loads in flight.
 // The forms at 512 are autotuner candidates.
@@ -44,12 +44,16 @@ constexpr int kBand32 = 5;
 constexpr int kBand16Pipe16 = 6;
 constexpr int kBand16Pipe32 = 7;
 constexpr int kBand16Pipe64 = 8;
+// kBandRegs: the register-ended kernel of the smaller sizes.
+constexpr int kBandRegs = 9;
 constexpr int band_pipe_columns(int form) {
     return form == kBand16Pipe16 ? 16 : form == kBand16Pipe32 ? 32 : form == kBand16Pipe64 ? 64 : 0;
 }
+// tw: the natural Ny-point table; table: the same in regs_table_index order.
 cudaError_t launch_columns_inverse_band(int ny, int nz, int zStride, int slots, int columns, DenseBins bins,
-                                        const int* band, const void* tw, int form, cudaStream_t s);
+                                        const int* band, const void* tw, const void* table, int form, cudaStream_t s);
 cudaError_t launch_columns_forward_band(int ny, int nz, int zStride, int slots, int columns, DenseBins bins,
-                                        const int* band, double scale, const void* tw, int form, cudaStream_t s);
+                                        const int* band, double scale, const void* tw, const void* table, int form,
+                                        cudaStream_t s);
 
 }  // namespace skb

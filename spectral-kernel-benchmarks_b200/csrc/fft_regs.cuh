@@ -85,6 +85,17 @@ __device__ __forceinline__ void dft_small(V* v) {
     if constexpr (R == 16) dft16<SIGN>(v);
 }
 
+// Exchange among threads (plane b of B, t) with b fastest, [position][plane]:
+// runs of B consecutive values, free of bank conflicts when B values fill an
+// access phase (128 bytes).
+template <typename V, int B>
+struct PlaneExchange {
+    V* x;  // this thread's plane
+    __device__ __forceinline__ void store(int i, V v) { x[i * B] = v; }
+    __device__ __forceinline__ V load(int i) const { return x[i * B]; }
+    __device__ __forceinline__ void fence() const { __syncthreads(); }
+};
+
 // One pass (sub-transforms of Ns points, radix R) on the thread's registers.
 // LDG: the table lies in global memory (read through __ldg), else anywhere.
 template <typename S, int N, int E, int SIGN, int Ns, bool LDG = true>

@@ -396,14 +396,6 @@ struct ColumnShape {
     static constexpr int kCtas = resident_ctas<T>(NT, kBytes, E);
 };
 
-template <typename V, int B>
-struct ColumnExchange {
-    V* x;  // this thread's plane of [position][plane]
-    __device__ __forceinline__ void store(int i, V v) { x[i * B] = v; }
-    __device__ __forceinline__ V load(int i) const { return x[i * B]; }
-    __device__ __forceinline__ void fence() const { __syncthreads(); }
-};
-
 // Input and output of a column kernel: plane p of a dense bin array, or level
 // p mod nz of retained view p / nz, so that chunks of planes run on across
 // views and only the last one is ragged.
@@ -419,7 +411,7 @@ __global__ void __launch_bounds__(ColumnShape<T, N>::NT, ColumnShape<T, N>::kCta
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int b = threadIdx.x % S::B;
     const int t = threadIdx.x / S::B;
-    ColumnExchange<V, S::B> xch{reinterpret_cast<V*>(smem_raw) + b};
+    PlaneExchange<V, S::B> xch{reinterpret_cast<V*>(smem_raw) + b};
     const long long kx = blockIdx.y;
     const long long p = (long long)blockIdx.x * S::B + b;
     const bool live = p < planes;
@@ -559,9 +551,8 @@ cudaError_t rows_forward_t(int nx, int ny, long long planes, int keep, const voi
         const cudaError_t err = allow_smem(kernel, S::kBytes);
         if (err != cudaSuccess) return err;
         const dim3 grid(unsigned((planes + S::B - 1) / S::B), unsigned(ny));
-        kernel<<<grid, S::NT, S::kBytes, stream>>>(ny, planes, keep, static_cast<const T*>(real), bins,
-                                                   static_cast<const cx<T>*>(twHalf),
-                                                   static_cast<const cx<T>*>(twFull));
+        kernel<<<grid, S::NT, S::kBytes, stream>>>(ny, planes, keep, static_cast<const T*>(real), bins, static_cast<const cx<T>*>(twHalf), static_cast<const cx<T>*>(twFull));
+        return cudaGetLastError();
     });
     return cudaGetLastError();
 }
@@ -582,9 +573,8 @@ cudaError_t rows_inverse_t(int nx, int ny, long long planes, int keep, DenseBins
         const cudaError_t err = allow_smem(kernel, S::kBytes);
         if (err != cudaSuccess) return err;
         const dim3 grid(unsigned((planes + S::B - 1) / S::B), unsigned(ny));
-        kernel<<<grid, S::NT, S::kBytes, stream>>>(ny, planes, keep, bins, static_cast<T*>(real),
-                                                   static_cast<const cx<T>*>(twHalf),
-                                                   static_cast<const cx<T>*>(twFull));
+        kernel<<<grid, S::NT, S::kBytes, stream>>>(ny, planes, keep, bins, static_cast<T*>(real), static_cast<const cx<T>*>(twHalf), static_cast<const cx<T>*>(twFull));
+        return cudaGetLastError();
     });
     return cudaGetLastError();
 }
@@ -598,8 +588,8 @@ cudaError_t columns_t(int ny, int columns, long long planes, DenseBins in, Dense
         const cudaError_t err = allow_smem(kernel, S::kBytes);
         if (err != cudaSuccess) return err;
         const dim3 grid(unsigned((planes + S::B - 1) / S::B), unsigned(columns));
-        kernel<<<grid, S::NT, S::kBytes, stream>>>(planes, in, out, nz, views, cells, T(scale),
-                                                   static_cast<const cx<T>*>(tw));
+        kernel<<<grid, S::NT, S::kBytes, stream>>>(planes, in, out, nz, views, cells, T(scale), static_cast<const cx<T>*>(tw));
+        return cudaGetLastError();
     });
     return cudaGetLastError();
 }

@@ -200,7 +200,7 @@ void HorizontalPlan::inverse_columns_band(DenseBins bins, int slots, int zStride
     if (!bandExact_ || p_ != Precision::f32 || !columns_warp_supported(static_cast<long long>(w_.ny)))
         throw Error(-3, "band column stage needs FP32, an exact retained band and Ny in [32, 512]");
     check_cuda(launch_columns_inverse_band(static_cast<int>(w_.ny), static_cast<int>(w_.nz), zStride, slots, keep_,
-                                           bins, band_.get<int>(), twCol_.get(), bandFormInverse_, s),
+                                           bins, band_.get<int>(), twCol_.get(), colTable_.get(), bandFormInverse_, s),
                "band inverse column kernel");
 }
 
@@ -208,7 +208,8 @@ void HorizontalPlan::forward_columns_band(DenseBins bins, int slots, double scal
     if (!bandExact_ || p_ != Precision::f32 || !columns_warp_supported(static_cast<long long>(w_.ny)))
         throw Error(-3, "band column stage needs FP32, an exact retained band and Ny in [32, 512]");
     check_cuda(launch_columns_forward_band(static_cast<int>(w_.ny), static_cast<int>(w_.nz), zStride, slots, keep_,
-                                           bins, band_.get<int>(), scale, twCol_.get(), bandFormForward_, s),
+                                           bins, band_.get<int>(), scale, twCol_.get(), colTable_.get(), bandFormForward_,
+                                           s),
                "band forward column kernel");
 }
 

@@ -42,3 +42,24 @@ def test_short_rows_match_fp64(n, nz, targets, members, planes):
         assert orc.rel_l2_error(one[:per], expected[:per]) <= 1e-6
         assert not one[per:].any()
     skb_cuda.tune_cache_clear()
+
+
+def test_register_band_columns_at_512():
+    """The register-ended band columns as a 512-point tuner choice (form 9)."""
+    skb_cuda.tune_cache_clear()
+    n, nz, members = 512, 9, 1
+    probe = skb_cuda.Flux(n, nz, members=members, mode=skb_cuda.FLUX_SPLIT_TF32X3)
+    rng = np.random.default_rng(9)
+    x = rng.uniform(-0.125, 0.125, probe.input_elements) + 1j * rng.uniform(-0.125, 0.125, probe.input_elements)
+    x = x.astype(np.complex64)
+    d_in = skb_cuda.DeviceArray.from_numpy(x)
+    d_out = skb_cuda.DeviceArray(probe.output_elements * 8)
+    band = [k for k in probe.autotune(d_in.ptr, d_out.ptr) if k.startswith("flux.columns_band.form")]
+    for key in band:
+        skb_cuda.tune_cache_store(key, 9, 0.0)
+    flux = skb_cuda.Flux(n, nz, members=members, mode=skb_cuda.FLUX_SPLIT_TF32X3)
+    expected = skb_cuda.Flux(n, nz, members=members).execute(x.astype(np.complex128))
+    flux.execute_device(d_in.ptr, d_out.ptr)
+    skb_cuda.synchronize()
+    assert orc.rel_l2_error(d_out.download(np.complex64, flux.output_elements), expected) <= 1e-6
+    skb_cuda.tune_cache_clear()
