@@ -16,6 +16,7 @@
 #include <algorithm>
 #include "async_copy.cuh"
 #include "fft_regs.cuh"
+#include "launch.cuh"
 
 namespace skb {
 namespace {
@@ -620,6 +621,7 @@ __global__ void __launch_bounds__(BandRegs<N>::NT, BandRegs<N>::kCtas)
     const int band = __ldg(bandOf + kx);
     const bool live = p < planes && static_cast<int>(p % zStride) < nz;
     const long long rowStride = bins.planes * bins.kxStride;
+    grid_wait();
     float2* const col = static_cast<float2*>(bins.data) + (live ? p : 0) + bins.planes * kx + rowStride * t;
     const long long step = rowStride * C::T;
     float2 v[C::E];
@@ -996,8 +998,8 @@ cudaError_t launch_band_regs(int nz, int zStride, int slots, int columns, DenseB
     if (err != cudaSuccess) return err;
     const long long planes = static_cast<long long>(slots) * zStride;
     const dim3 grid(unsigned((planes + C::B - 1) / C::B), unsigned(columns));
-    kernel<<<grid, C::NT, C::kBytes, s>>>(nz, zStride, planes, bins, band, scale, static_cast<const float2*>(table));
-    return cudaGetLastError();
+    return launch_chained(kernel, grid, C::NT, C::kBytes, s, nz, zStride, planes, bins, band, scale,
+                          static_cast<const float2*>(table));
 }
 
 cudaError_t inverse_band_512(int nz, int zStride, int slots, int columns, DenseBins bins, const int* band, const void* tw,

@@ -27,6 +27,7 @@
 
 #include "async_copy.cuh"
 #include "fft_regs.cuh"
+#include "launch.cuh"
 #include "tensor_map.hpp"
 
 namespace skb {
@@ -532,6 +533,7 @@ __global__ void __launch_bounds__(M / 16 * B, MINB)
         return true;
     };
 
+    grid_wait();
     if constexpr (TMA) __syncthreads();  // barrier init and zero rows before the first copy and reads
     for (int f = 0; f < NST - 1 && f < a.fieldsIn; ++f) issue(f);
     V u[16], v[16], w[16];
@@ -609,8 +611,7 @@ cudaError_t launch_pair(const RowFluxArgs& a, cudaStream_t stream) {
     }
     const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
     if (err != cudaSuccess) return err;
-    kernel<<<grid, M / 16 * B, bytes, stream>>>(a, map);
-    return cudaGetLastError();
+    return launch_chained(kernel, grid, M / 16 * B, bytes, stream, a, map);
 }
 
 template <int NS>

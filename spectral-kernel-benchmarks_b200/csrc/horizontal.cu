@@ -5,6 +5,7 @@
 #include "horizontal.hpp"
 
 #include "fft_regs.cuh"
+#include "launch.cuh"
 
 namespace skb {
 namespace {
@@ -115,6 +116,7 @@ __global__ void __launch_bounds__(RowShape<T, M>::NT, RowShape<T, M>::kCtas)
     const long long p0 = (long long)blockIdx.x * S::B;
     const int y = blockIdx.y;
     V v[S::E];
+    grid_wait();
     {
         const int t = tid % S::TPR;
         const int b = tid / S::TPR;
@@ -222,6 +224,7 @@ __global__ void __launch_bounds__(RowShape<T, M>::NT, RowShape<T, M>::kCtas)
     const long long p0 = (long long)blockIdx.x * S::B;
     const int y = blockIdx.y;
     V v[S::E];
+    grid_wait();
     {
         const int b = tid % S::B;
         const int g = tid / S::B;
@@ -428,6 +431,7 @@ __global__ void __launch_bounds__(ColumnShape<T, N>::NT, ColumnShape<T, N>::kCta
         int cell[S::E];
 #pragma unroll
         for (int e = 0; e < S::E; ++e) cell[e] = __ldg(map + S::TPC * e);
+        grid_wait();
 #pragma unroll
         for (int e = 0; e < S::E; ++e)
             v[e] = live && cell[e] >= 0 ? view_load<T>(view, cell[e] >> 1, z) : V{T(0), T(0)};
@@ -435,6 +439,7 @@ __global__ void __launch_bounds__(ColumnShape<T, N>::NT, ColumnShape<T, N>::kCta
         for (int e = 0; e < S::E; ++e)
             if (cell[e] & 1) v[e] = cconj(v[e]);
     } else {
+        grid_wait();
         const V* src =
             reinterpret_cast<const V*>(in.data) + in.offset(live ? p : 0) + in.planes * (kx + in.kxStride * t);
         const long long step = in.planes * in.kxStride * S::TPC;
@@ -551,8 +556,8 @@ cudaError_t rows_forward_t(int nx, int ny, long long planes, int keep, const voi
         const cudaError_t err = allow_smem(kernel, S::kBytes);
         if (err != cudaSuccess) return err;
         const dim3 grid(unsigned((planes + S::B - 1) / S::B), unsigned(ny));
-        kernel<<<grid, S::NT, S::kBytes, stream>>>(ny, planes, keep, static_cast<const T*>(real), bins, static_cast<const cx<T>*>(twHalf), static_cast<const cx<T>*>(twFull));
-        return cudaGetLastError();
+        return launch_chained(kernel, grid, S::NT, S::kBytes, stream, ny, planes, keep, static_cast<const T*>(real),
+                              bins, static_cast<const cx<T>*>(twHalf), static_cast<const cx<T>*>(twFull));
     });
     return cudaGetLastError();
 }
@@ -573,8 +578,8 @@ cudaError_t rows_inverse_t(int nx, int ny, long long planes, int keep, DenseBins
         const cudaError_t err = allow_smem(kernel, S::kBytes);
         if (err != cudaSuccess) return err;
         const dim3 grid(unsigned((planes + S::B - 1) / S::B), unsigned(ny));
-        kernel<<<grid, S::NT, S::kBytes, stream>>>(ny, planes, keep, bins, static_cast<T*>(real), static_cast<const cx<T>*>(twHalf), static_cast<const cx<T>*>(twFull));
-        return cudaGetLastError();
+        return launch_chained(kernel, grid, S::NT, S::kBytes, stream, ny, planes, keep, bins, static_cast<T*>(real),
+                              static_cast<const cx<T>*>(twHalf), static_cast<const cx<T>*>(twFull));
     });
     return cudaGetLastError();
 }
@@ -588,8 +593,8 @@ cudaError_t columns_t(int ny, int columns, long long planes, DenseBins in, Dense
         const cudaError_t err = allow_smem(kernel, S::kBytes);
         if (err != cudaSuccess) return err;
         const dim3 grid(unsigned((planes + S::B - 1) / S::B), unsigned(columns));
-        kernel<<<grid, S::NT, S::kBytes, stream>>>(planes, in, out, nz, views, cells, T(scale), static_cast<const cx<T>*>(tw));
-        return cudaGetLastError();
+        return launch_chained(kernel, grid, S::NT, S::kBytes, stream, planes, in, out, nz, views, cells, T(scale),
+                              static_cast<const cx<T>*>(tw));
     });
     return cudaGetLastError();
 }

@@ -5,6 +5,7 @@
 #include "pipeline.hpp"
 
 #include "fft_device.cuh"
+#include "launch.cuh"
 
 namespace skb {
 namespace {
@@ -12,6 +13,7 @@ namespace {
 template <typename T>
 __global__ void modal_work_kernel(const T* __restrict__ weights, const cx<T>* __restrict__ in, cx<T>* out,
                                   long long count) {
+    grid_wait();
     const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
     for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += stride) {
         const T w = __ldg(weights + i);
@@ -28,12 +30,12 @@ cudaError_t launch_modal_work(Precision p, const void* weights, const void* in, 
     const int threads = 256;
     const long long blocks = std::min<long long>((count + threads - 1) / threads, 148LL * 16);
     if (p == Precision::f64)
-        modal_work_kernel<double><<<unsigned(blocks), threads, 0, s>>>(
-            static_cast<const double*>(weights), static_cast<const double2*>(in), static_cast<double2*>(out), count);
-    else
-        modal_work_kernel<float><<<unsigned(blocks), threads, 0, s>>>(
-            static_cast<const float*>(weights), static_cast<const float2*>(in), static_cast<float2*>(out), count);
-    return cudaGetLastError();
+        return launch_chained(modal_work_kernel<double>, dim3(unsigned(blocks)), threads, 0, s,
+                              static_cast<const double*>(weights), static_cast<const double2*>(in),
+                              static_cast<double2*>(out), count);
+    return launch_chained(modal_work_kernel<float>, dim3(unsigned(blocks)), threads, 0, s,
+                          static_cast<const float*>(weights), static_cast<const float2*>(in), static_cast<float2*>(out),
+                          count);
 }
 
 }  // namespace skb

@@ -5,6 +5,8 @@
 
 #include "pointwise.hpp"
 
+#include "launch.cuh"
+
 namespace skb {
 namespace {
 
@@ -17,6 +19,7 @@ __global__ void pointwise_kernel(long long volume, T scale, const T* __restrict_
     const T* qx = derivative;
     const T* qy = derivative + volume;
     const T* qz = derivative + 2 * volume;
+    grid_wait();
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < volume; i += stride)
         target[i] = -scale * (u[i] * qx[i] + v[i] * qy[i] + w[i] * qz[i]);
@@ -26,6 +29,7 @@ template <typename T, typename V2>
 __global__ void pointwise_vec2_kernel(long long pairs, T scale, const V2* __restrict__ u, const V2* __restrict__ v,
                                       const V2* __restrict__ w, const V2* __restrict__ qx,
                                       const V2* __restrict__ qy, const V2* __restrict__ qz, V2* __restrict__ target) {
+    grid_wait();
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < pairs; i += stride) {
         const V2 a = u[i], b = v[i], c = w[i], x = qx[i], y = qy[i], z = qz[i];
@@ -49,16 +53,17 @@ cudaError_t launch_t(long long volume, double scale, const void* shared, const v
     if (aligned) {
         const long long pairs = volume / 2;
         const long long blocks = std::min<long long>((pairs + threads - 1) / threads, (long long)smCount * 16);
-        pointwise_vec2_kernel<T, V2><<<unsigned(std::max(1LL, blocks)), threads, 0, stream>>>(
-            pairs, T(scale), reinterpret_cast<const V2*>(s), reinterpret_cast<const V2*>(s + volume),
+        return launch_chained(
+            pointwise_vec2_kernel<T, V2>, dim3(unsigned(std::max(1LL, blocks))), threads, 0, stream, pairs, T(scale),
+            reinterpret_cast<const V2*>(s), reinterpret_cast<const V2*>(s + volume),
             reinterpret_cast<const V2*>(s + 2 * volume), reinterpret_cast<const V2*>(d),
             reinterpret_cast<const V2*>(d + volume), reinterpret_cast<const V2*>(d + 2 * volume),
             reinterpret_cast<V2*>(t));
     } else {
         const long long blocks = std::min<long long>((volume + threads - 1) / threads, (long long)smCount * 16);
-        pointwise_kernel<T><<<unsigned(std::max(1LL, blocks)), threads, 0, stream>>>(volume, T(scale), s, d, t);
+        return launch_chained(pointwise_kernel<T>, dim3(unsigned(std::max(1LL, blocks))), threads, 0, stream, volume,
+                              T(scale), s, d, t);
     }
-    return cudaGetLastError();
 }
 
 }  // namespace

@@ -37,6 +37,7 @@
 #include <algorithm>
 #include <cstdint>
 
+#include "launch.cuh"
 #include "vertical.hpp"
 
 namespace skb {
@@ -419,6 +420,7 @@ __global__ void __launch_bounds__(kPipeThreads, 1) tc_gemm_pipe_kernel(TcGemmArg
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = st->tmem;
+    grid_wait();
     bool failed = false;
     // A bounded wait that expired: stop this role and make the others stop too.
     auto fail = [&] {
@@ -850,8 +852,7 @@ cudaError_t launch_np(const TcGemmArgs& args, cudaStream_t stream) {
         cudaDeviceGetAttribute(&smCount[device], cudaDevAttrMultiProcessorCount, device);
     const int sms = (device >= 0 && device < 64 && smCount[device] > 0) ? smCount[device] : 148;
     const int grid = args.ctaFirst != nullptr ? args.ctas : std::min(args.units, sms);
-    kernel<<<grid, kPipeThreads, bytes, stream>>>(args);
-    return cudaGetLastError();
+    return launch_chained(kernel, dim3(unsigned(grid)), kPipeThreads, bytes, stream, args);
 }
 }  // namespace
 

@@ -23,6 +23,7 @@
 // 15-field inverse 2.14 -> 1.43 ms, 4-field forward 0.82 -> 0.42 ms.  Persistent
 // CTAs with the copies running across tiles: 77 us, and 1 % slower at 512^2.
 
+#include "launch.cuh"
 #include "vertical_device.cuh"
 
 namespace skb {
@@ -162,6 +163,7 @@ __global__ void __launch_bounds__(kThreads, resident<MH>())
 #pragma unroll
         for (int n = 0; n < 2; ++n) acc[i][n][0] = acc[i][n][1] = 0.0;
 
+    grid_wait();
     issue(0, 0);
     for (int c = 0; c < chunks; ++c) {
         if (c + 1 < chunks) {
@@ -228,8 +230,8 @@ cudaError_t launch_mh(int R, int S, const double* images, const GroupTiles& tile
         const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
         if (err != cudaSuccess) return err;
     }
-    kernel<<<tiles.tiles, kThreads, bytes, stream>>>(R, S, images, tiles, in, out, ib, ob);
-    return cudaGetLastError();
+    return launch_chained(kernel, dim3(unsigned(tiles.tiles)), kThreads, bytes, stream, R, S, images, tiles, in, out, ib,
+                          ob);
 }
 
 }  // namespace
