@@ -163,6 +163,20 @@ FluxPipeline::FluxPipeline(const FluxConfig& cfg) : cfg_(cfg) {
     // Staged: 2 GEMMs, 2 launches per inverse / forward horizontal, members pointwise per target.
     // Fused: GEMM, embed+columns, fused rows, columns+retention, GEMM.  With
     // operator families each GEMM is one launch per family.
+    if (fused_ && dense_ && cfg.n == 512) {
+        // Forms of an untuned handle, the autotuner's usual picks.  Rows: two
+        // planes per warp, three CTAs per SM, TMA stages (one member, Nz 129:
+        // 997 us warp per plane -> 765).  Columns: the pipelined form walking
+        // 16 columns from 128 chunks of 16 planes on, where its one CTA per SM
+        // has several waves (15 slots of 129, one member: direct 697 us, 16
+        // planes 570, pipelined 532; 12 slots of 33: 150, 144, 165); forward
+        // from there on either 16-plane form, register-ended below (4 slots of
+        // 129: 138 us against 146 and 156).
+        rowsPairs_ = 2;
+        rowsTma_ = 1;
+        const std::uint64_t inChunks = cfg.members * fieldsIn_ * zStride_ / 16;
+        horizontal_->set_band_forms(inChunks >= 127 ? kBand16Pipe16 : kBand16, kBandRegs);
+    }
     launches_ = (fused_ ? 5 : 2 + 2 + cfg.targets * (2 + cfg.members + 2)) + (families_ ? 2 : 0);
     apply_tuned(nullptr, nullptr, nullptr, nullptr);
 }
