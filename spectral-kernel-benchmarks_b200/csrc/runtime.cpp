@@ -47,7 +47,7 @@ int sm_count() {
 
 size_t element_bytes(Precision p) { return p == Precision::f64 ? sizeof(double) : sizeof(float); }
 
-std::vector<double> regs_table(const std::vector<double>& natural, int perThread, int first = 0) {
+std::vector<double> regs_table(const std::vector<double>& natural, int perThread, int first) {
     const int n = static_cast<int>(natural.size() / 2);
     std::vector<double> out;
     for (int i = 0; i < regs_table_size(n, perThread, first); ++i) {

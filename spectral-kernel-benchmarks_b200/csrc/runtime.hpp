@@ -84,6 +84,9 @@ DeviceBuffer upload_vector(const std::vector<T>& v) {
 int sm_count();
 size_t element_bytes(Precision p);
 
+// A natural table of n twiddles (re, im pairs) in regs_table_index order.
+std::vector<double> regs_table(const std::vector<double>& natural, int perThread, int first = 0);
+
 // Upload a double table in the plan's precision.
 DeviceBuffer upload_real_table(const std::vector<double>& values, Precision p);
 

@@ -4,17 +4,25 @@
 // of the column's even extension e (e_z = e_{L-z} = x_z); a DST-I of the
 // interior is i times the DFT of the odd extension (o_z = -o_{L-z} = x_z,
 // o_0 = o_{nz-1} = 0).  Both hold for complex columns because the transform
-// matrices are real.  Each warp walks (row, channel) columns with a grid
-// stride: it holds the next column's values in registers while it writes the
-// current one's extension into its shared-memory slot, runs warp_fft and
-// writes the nz results back over the column (all reads of a column finish
-// before its first write, so the transform is in place).  Columns are
-// contiguous in HBM, so each warp moves whole sectors; the bound is HBM
-// traffic (one read and one write of every transformed value).
+// matrices are real.
+//
+// Up to L = 512 the transform is register-ended (fft_regs.cuh): T = L/E lanes of
+// a warp share a column, lane t loads the extension's elements t + T e straight
+// from the column (the upper half mirrored, from lines the lower half has just
+// read), and stores the results k = t + T e <= nz-1; the exchange between the two
+// passes (two at L = 512) is the only shared-memory traffic.  All of a column is
+// read before its first store, so the transform is in place.  Bound: HBM (one
+// read and one write of every transformed value), then load latency.  FP64,
+// 45,765 rows of 3 channels, nz 129 (567 MB per transform): 284 -> 110 us (5.15 TB/s) against
+// the warp-per-column kernel with the extension and three passes in shared
+// memory, which ran the L1 pipe at 91 % and HBM at 21 %; that kernel stays for
+// L = 1024, whose 64 lanes would not fit a warp.
 
 #include <algorithm>
 
-#include "fft_device.cuh"
+#include "fft_regs.cuh"
+#include "horizontal.hpp"
+#include "launch.cuh"
 #include "type1.hpp"
 
 namespace skb {
@@ -39,6 +47,66 @@ __device__ __forceinline__ void store_result(cx<T>* col, int k, cx<T> y, int M, 
     col[k] = y;
 }
 
+template <int L>
+struct Type1Regs {
+    static constexpr int E = regs_per_thread(L);
+    static constexpr int TPC = L / E;            // lanes per column
+    static constexpr int NT = 128;
+    static constexpr int COLS = NT / TPC;        // columns per CTA
+    static constexpr int XP = L + L / E;         // one spare slot per E spreads the first pass's stores
+    static_assert(TPC <= 32 && E % 2 == 0, "a column's lanes form (part of) one warp");
+};
+
+template <typename V, int E>
+struct LaneExchange {
+    V* x;
+    __device__ __forceinline__ void store(int i, V v) { x[i + i / E] = v; }
+    __device__ __forceinline__ V load(int i) const { return x[i + i / E]; }
+    __device__ __forceinline__ void fence() const { __syncwarp(); }
+};
+
+template <typename T, int L>
+__global__ void __launch_bounds__(Type1Regs<L>::NT) type1_regs_kernel(cx<T>* __restrict__ data, long long seqs,
+                                                                      int storage, int first, int channels,
+                                                                      unsigned dstMask, bool normalize,
+                                                                      const cx<T>* __restrict__ table) {
+    using V = cx<T>;
+    using C = Type1Regs<L>;
+    constexpr int M = L / 2, nz = M + 1;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int t = threadIdx.x % C::TPC;
+    const int local = threadIdx.x / C::TPC;
+    const long long seq = static_cast<long long>(blockIdx.x) * C::COLS + local;
+    const bool live = seq < seqs;
+    const long long row = live ? seq / channels : 0;
+    const int c = live ? static_cast<int>(seq - row * channels) : 0;
+    const bool sine = (dstMask >> c) & 1u;
+    V* col = data + (row * storage + first + c) * nz;
+    V v[C::E];
+    grid_wait();
+    // Elements below M are the column's, those from M on are its values L - i
+    // (negated in the odd extension, whose elements 0 and M are zero).
+    const T mirror = sine ? T(-1) : T(1);
+#pragma unroll
+    for (int e = 0; e < C::E; ++e) {
+        const int i = t + C::TPC * e;
+        V x = live ? col[e < C::E / 2 ? i : L - i] : V{T(0), T(0)};
+        if (e >= C::E / 2) x = V{mirror * x.x, mirror * x.y};
+        if ((e == 0 || e == C::E / 2) && t == 0 && sine) x = V{T(0), T(0)};
+        v[e] = x;
+    }
+    LaneExchange<V, C::E> xch{reinterpret_cast<V*>(smem_raw) + local * C::XP};
+    fft_regs<T, L, C::E, -1>(v, t, table, xch);
+    if (!live) return;
+#pragma unroll
+    for (int e = 0; e <= C::E / 2; ++e) {
+        const int k = t + C::TPC * e;
+        const V y = sine ? V{-v[e].y, v[e].x} : v[e];  // i X_k
+        if (k <= M) store_result<T>(col, k, y, M, sine, normalize);
+    }
+}
+
+// Warp per column, the extension in shared memory (L = 1024).
 template <typename T, int L>
 __global__ void __launch_bounds__(kWarps * 32) type1_fft_kernel(cx<T>* __restrict__ data, long long seqs, int storage,
                                                                 int first, int channels, unsigned dstMask,
@@ -197,21 +265,34 @@ cudaError_t launch_fft(cx<T>* data, long long seqs, int storage, int first, int 
     return cudaGetLastError();
 }
 
+template <typename T, int L>
+cudaError_t launch_regs(cx<T>* data, long long seqs, int storage, int first, int channels, unsigned mask, bool norm,
+                        const cx<T>* table, cudaStream_t s) {
+    using C = Type1Regs<L>;
+    const size_t bytes = C::TPC > 1 ? sizeof(cx<T>) * C::COLS * C::XP : 0;
+    auto kernel = type1_regs_kernel<T, L>;
+    const long long blocks = (seqs + C::COLS - 1) / C::COLS;
+    if (blocks > 0x7FFFFFFFLL) return cudaErrorInvalidValue;
+    return launch_chained(kernel, dim3(static_cast<unsigned>(blocks)), C::NT, bytes, s, data, seqs, storage, first,
+                          channels, mask, norm, table);
+}
+
 template <typename T>
 cudaError_t launch_t(void* data, long long rows, int nz, int storage, int first, int channels, unsigned mask,
-                     bool norm, const void* twv, cudaStream_t s) {
+                     bool norm, const void* twv, const void* tablev, cudaStream_t s) {
     auto* d = static_cast<cx<T>*>(data);
     const auto* tw = static_cast<const cx<T>*>(twv);
+    const auto* table = static_cast<const cx<T>*>(tablev);
     const long long seqs = rows * channels;
     if (seqs == 0) return cudaSuccess;
     switch (2 * (nz - 1)) {
-        case 8: return launch_fft<T, 8>(d, seqs, storage, first, channels, mask, norm, tw, s);
-        case 16: return launch_fft<T, 16>(d, seqs, storage, first, channels, mask, norm, tw, s);
-        case 32: return launch_fft<T, 32>(d, seqs, storage, first, channels, mask, norm, tw, s);
-        case 64: return launch_fft<T, 64>(d, seqs, storage, first, channels, mask, norm, tw, s);
-        case 128: return launch_fft<T, 128>(d, seqs, storage, first, channels, mask, norm, tw, s);
-        case 256: return launch_fft<T, 256>(d, seqs, storage, first, channels, mask, norm, tw, s);
-        case 512: return launch_fft<T, 512>(d, seqs, storage, first, channels, mask, norm, tw, s);
+        case 8: return launch_regs<T, 8>(d, seqs, storage, first, channels, mask, norm, table, s);
+        case 16: return launch_regs<T, 16>(d, seqs, storage, first, channels, mask, norm, table, s);
+        case 32: return launch_regs<T, 32>(d, seqs, storage, first, channels, mask, norm, table, s);
+        case 64: return launch_regs<T, 64>(d, seqs, storage, first, channels, mask, norm, table, s);
+        case 128: return launch_regs<T, 128>(d, seqs, storage, first, channels, mask, norm, table, s);
+        case 256: return launch_regs<T, 256>(d, seqs, storage, first, channels, mask, norm, table, s);
+        case 512: return launch_regs<T, 512>(d, seqs, storage, first, channels, mask, norm, table, s);
         case 1024: return launch_fft<T, 1024>(d, seqs, storage, first, channels, mask, norm, tw, s);
         default: break;
     }
@@ -237,11 +318,11 @@ bool type1_uses_fft(int nz) {
 }
 
 cudaError_t launch_type1(bool f64, void* data, long long rows, int nz, int storageChannels, int first, int channels,
-                         unsigned dstMask, bool normalize, const void* tw, cudaStream_t s) {
+                         unsigned dstMask, bool normalize, const void* tw, const void* table, cudaStream_t s) {
     if (nz < 3 || channels <= 0 || first < 0 || first + channels > storageChannels || channels > 32)
         return cudaErrorInvalidValue;
-    return f64 ? launch_t<double>(data, rows, nz, storageChannels, first, channels, dstMask, normalize, tw, s)
-               : launch_t<float>(data, rows, nz, storageChannels, first, channels, dstMask, normalize, tw, s);
+    return f64 ? launch_t<double>(data, rows, nz, storageChannels, first, channels, dstMask, normalize, tw, table, s)
+               : launch_t<float>(data, rows, nz, storageChannels, first, channels, dstMask, normalize, tw, table, s);
 }
 
 cudaError_t launch_type1_normalize(bool f64, void* data, long long rows, int nz, int storageChannels, int first,

@@ -20,9 +20,10 @@
 namespace skb {
 
 // tw: L = 2(nz-1) complex twiddles exp(-2 pi i m / L), m in [0, L), of the
-// handle's precision.
+// handle's precision; table: the same in regs_table_index order of
+// (L, regs_per_thread(L)), read for the power-of-two L up to 512.
 cudaError_t launch_type1(bool f64, void* data, long long rows, int nz, int storageChannels, int first, int channels,
-                         unsigned dstMask, bool normalize, const void* tw, cudaStream_t s);
+                         unsigned dstMask, bool normalize, const void* tw, const void* table, cudaStream_t s);
 // The normalisation alone (the reference's separate adapter pass).
 cudaError_t launch_type1_normalize(bool f64, void* data, long long rows, int nz, int storageChannels, int first,
                                    int channels, unsigned dstMask, cudaStream_t s);
