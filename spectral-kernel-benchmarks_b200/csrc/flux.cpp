@@ -10,6 +10,11 @@
 
 namespace skb {
 
+// A member's result is the same alone and in a batch, so its GEMM form may not
+// depend on the handle's batch: it is chosen for batches of 8, the largest that the
+// repository's workloads run.
+constexpr std::uint64_t kGemmBatch = 8;
+
 FluxPipeline::FluxPipeline(const FluxConfig& cfg) : cfg_(cfg) {
     if (cfg.n < 2 || cfg.nz < 2) throw Error(-1, "flux requires n >= 2 and Nz >= 2");
     if (cfg.targets != 4 && cfg.targets != 3) throw Error(-1, "flux targets must be 4 (15 -> 4) or 3 (12 -> 3)");
@@ -77,9 +82,9 @@ FluxPipeline::FluxPipeline(const FluxConfig& cfg) : cfg_(cfg) {
                                                    maxPlanes);
     if (!families_) {
         inverseGemm_ = std::make_unique<VerticalPlan>(gp, static_cast<int>(cfg.nz), static_cast<int>(nj_), groups,
-                                                      fieldsIn_, cfg.members, fam.inverse);
+                                                      fieldsIn_, cfg.members, fam.inverse, kGemmBatch);
         forwardGemm_ = std::make_unique<VerticalPlan>(gp, static_cast<int>(nj_), static_cast<int>(cfg.nz), groups,
-                                                      cfg.targets, cfg.members, fam.forward);
+                                                      cfg.targets, cfg.members, fam.forward, kGemmBatch);
     } else {
         const FluxFamilies& F = *cfg.families;
         for (int f = 0; f < 2; ++f) {
@@ -90,13 +95,15 @@ FluxPipeline::FluxPipeline(const FluxConfig& cfg) : cfg_(cfg) {
                 if (F.targetFamily[t] == f) out.push_back(static_cast<int>(t));
             if (!in.empty()) {
                 inverseFamily_[f].plan = std::make_unique<VerticalPlan>(
-                    gp, static_cast<int>(cfg.nz), static_cast<int>(nj_), groups, in.size(), cfg.members, F.inverse[f]);
+                    gp, static_cast<int>(cfg.nz), static_cast<int>(nj_), groups, in.size(), cfg.members, F.inverse[f],
+                    kGemmBatch);
                 inverseFamily_[f].fieldMap = upload_vector(in);
                 inverseFamily_[f].fields = static_cast<int>(in.size());
             }
             if (!out.empty()) {
                 forwardFamily_[f].plan = std::make_unique<VerticalPlan>(
-                    gp, static_cast<int>(nj_), static_cast<int>(cfg.nz), groups, out.size(), cfg.members, F.forward[f]);
+                    gp, static_cast<int>(nj_), static_cast<int>(cfg.nz), groups, out.size(), cfg.members, F.forward[f],
+                    kGemmBatch);
                 forwardFamily_[f].fieldMap = upload_vector(out);
                 forwardFamily_[f].fields = static_cast<int>(out.size());
             }

@@ -275,8 +275,39 @@ void HorizontalPlan::embed_dense(const ViewSet& views, void* wvm, std::uint64_t 
                "embedding kernel");
 }
 
+// Which split-TF32x3 form serves a plan: tiles of 32 columns on mma.sync
+// (vertical_tf32.cu) or the tcgen05 pipeline (tc_gemm.cu).  The estimates, in
+// microseconds, are fits to both kernels at the 22 shapes of 64^2 to 512^2, Nz 17 to
+// 129 and 1 to 8 members that were timed (within 12 % where the time is above 50 us):
+// mma.sync pays by column, 0.18 ns for its loads and stores and 14 ps per 16 x 8 block
+// of the padded matrix; the pipeline pays by 64-column tile on one of 148 SMs, however
+// full the tile.  Measured, mma.sync / tcgen05 us: 256^2, Nz 65: 3-field forward of
+// one member 41 / 71, of 4 97 / 96, 4 fields of 8 223 / 174, 12-field inverse 95 / 81;
+// 512^2, Nz 129: 4-field forward 320 / 401, of 2 members 569 / 449, 15-field inverse
+// 1000 / 472; 128^2, Nz 33: 3-field forward 12 / 20, of 8 members 29 / 36, 12-field
+// inverse 18 / 22, of 8 members 91 / 75.  The pipeline has to be 10 % behind.
+//
+// The two forms round differently, so a plan whose members may run in batches of any
+// size must choose the same form for every batch: `batch` is the size that the choice
+// is made for, whatever the plan's own.
+static bool tf32_small_groups(int R, int S, const std::vector<ModeGroup>& groups, std::uint64_t fields,
+                              std::uint64_t batch) {
+    if (R > kGemmTf32MaxRows) return false;
+    double columns = 0.0, tiles = 0.0;
+    for (const auto& g : groups) {
+        const std::uint64_t c = g.count * fields * batch;
+        columns += static_cast<double>(c);
+        tiles += static_cast<double>((c + 63) / 64);
+    }
+    const int rows = (R + 15) / 16;
+    const double small = 8.2 + columns * (0.18e-3 + 14e-6 * rows * ((S + 7) / 8));
+    const double pipeline = 10.8 + tiles * (0.28 + 0.23 * rows + 1.1 * ((S + 31) / 32)) / 148.0;
+    return 1.1 * small < pipeline;
+}
+
 VerticalPlan::VerticalPlan(GemmPrecision p, int rowsOut, int inner, const std::vector<ModeGroup>& groups,
-                           std::uint64_t fields, std::uint64_t members, const std::vector<double>& natural)
+                           std::uint64_t fields, std::uint64_t members, const std::vector<double>& natural,
+                           std::uint64_t batch)
     : p_(p), R_(rowsOut), S_(inner) {
     if (groups.empty() || fields == 0 || members == 0) throw Error(-1, "Vertical GEMM requires groups and fields.");
     const auto matrixElems = static_cast<std::uint64_t>(rowsOut) * inner;
@@ -300,6 +331,11 @@ VerticalPlan::VerticalPlan(GemmPrecision p, int rowsOut, int inner, const std::v
             throw Error(-2, "unsupported: tensor-core GEMM needs the padded group matrix and two data stages in "
                             "227 KB of shared memory (R=" + std::to_string(rowsOut) + ", S=" + std::to_string(inner) +
                             ")");
+        error_.allocate(sizeof(int));
+        check_cuda(cudaMemset(error_.get(), 0, sizeof(int)), "cudaMemset");
+        smallGroups_ = p == GemmPrecision::tf32x3 && tf32_small_groups(rowsOut, inner, groups, fields, batch);
+    }
+    if (tensor_core() && !smallGroups_) {
         // FP32 matrices (one, if common to all groups) -> the kernel's
         // operand images, split into TF32 hi/lo or BF16 h/m/l and swizzled
         // once here.
@@ -321,8 +357,6 @@ VerticalPlan::VerticalPlan(GemmPrecision p, int rowsOut, int inner, const std::v
         build_units(tc_gemm_unit_tiles());
         groupColumns_ = upload_vector(gc);
         groupFirst_ = upload_vector(gf);
-        error_.allocate(sizeof(int));
-        check_cuda(cudaMemset(error_.get(), 0, sizeof(int)), "cudaMemset");
         return;
     }
 
@@ -371,6 +405,16 @@ VerticalPlan::VerticalPlan(GemmPrecision p, int rowsOut, int inner, const std::v
             }
         matrices_ = upload_vector(images);
         matrixStride_ = common ? 0 : static_cast<long long>(imageElems);
+    } else if (smallGroups_) {
+        const std::uint64_t imageElems = static_cast<std::uint64_t>(rowsOut) * gemm_tf32_row(inner);
+        const DeviceBuffer staged = upload_vector(std::vector<float>(natural.begin(), natural.end()));
+        matrices_.allocate(groupsCount * imageElems * sizeof(float));
+        check_cuda(gemm_tf32_build_images(staged.get<float>(), static_cast<long long>(groupsCount), rowsOut, inner,
+                                          matrices_.get<float>(), nullptr),
+                   "split-TF32x3 GEMM images");
+        check_cuda(cudaStreamSynchronize(nullptr), "split-TF32x3 GEMM images");
+        matrixStride_ = common ? 0 : static_cast<long long>(imageElems);
+        unitTiles_ = tc_gemm_unit_tiles();
     } else {
         // The FP32 form reads the transposed matrices At[g][s][r].
         std::vector<float> At(groupsCount * matrixElems);
@@ -481,7 +525,10 @@ void VerticalPlan::build_units(int tiles) {
 
 void VerticalPlan::set_unit_tiles(int tiles) {
     if (!tensor_core()) throw Error(-3, "work-unit size applies to the tensor-core forms only");
-    if (tiles != unitTiles_) build_units(tiles);
+    if (smallGroups_)
+        unitTiles_ = tiles;  // no units: the choice has no effect
+    else if (tiles != unitTiles_)
+        build_units(tiles);
 }
 
 std::uint64_t VerticalPlan::persistentBytes() const {
@@ -497,9 +544,9 @@ void VerticalPlan::execute(ComplexOperand in, ComplexOperand out, cudaStream_t s
                            const BinBoundary* inBins, const BinBoundary* outBins) const {
     if (members == 0) members = members_;
     if (members > members_) throw Error(-1, "more ensemble members than the plan was built for");
-    if (tensor_core()) {
-        if (in.im != nullptr || out.im != nullptr)
-            throw Error(-3, "the tensor-core GEMM form takes interleaved complex operands");
+    if (tensor_core() && (in.im != nullptr || out.im != nullptr))
+        throw Error(-3, "the tensor-core GEMM form takes interleaved complex operands");
+    if (tensor_core() && !smallGroups_) {
         const UnitTable& table = unitTables_[members - 1];
         TcGemmArgs a{};
         a.B = matrices_.get<unsigned char>();
@@ -542,6 +589,13 @@ void VerticalPlan::execute(ComplexOperand in, ComplexOperand out, cudaStream_t s
     if (outBins != nullptr) {
         ob = *outBins;
         ob.memberColumns = memberColumns_;
+    }
+    if (smallGroups_) {
+        check_cuda(launch_grouped_gemm_tf32(R_, S_, matrices_.get<float>(), t, static_cast<const float2*>(in.re),
+                                            static_cast<float2*>(out.re), ib, ob, error_.get<int>(),
+                                            expireWaitForTest_, s),
+                   "split-TF32x3 grouped vertical GEMM kernel");
+        return;
     }
     check_cuda(launch_grouped_gemm(p_, R_, S_, matrices_.get(), t, in, out, s, inBins ? &ib : nullptr,
                                    outBins ? &ob : nullptr),

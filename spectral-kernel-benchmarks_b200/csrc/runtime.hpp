@@ -171,9 +171,12 @@ class VerticalPlan {
 public:
     // rowsOut x inner matrices per group, natural layout A[g][r][s]
     // (forward: F[g][j][z], inverse: I[g][z][j]); one matrix for all groups
-    // when `natural` holds a single rowsOut x inner block.
+    // when `natural` holds a single rowsOut x inner block.  `batch`: the batch of
+    // members that the split-TF32x3 form is chosen for; callers whose members also
+    // run in other batches give one value for all of them.
     VerticalPlan(GemmPrecision p, int rowsOut, int inner, const std::vector<ModeGroup>& groups,
-                 std::uint64_t fields, std::uint64_t members, const std::vector<double>& natural);
+                 std::uint64_t fields, std::uint64_t members, const std::vector<double>& natural,
+                 std::uint64_t batch = 1);
     // `members` <= the capacity given at construction (0 = all): the first
     // `members` ensemble members are computed.
     // inBins / outBins (tensor-core form only): operands in the fused flux's
@@ -217,6 +220,7 @@ private:
     };
     std::vector<TileTable> tileTables_;
     std::vector<int> tilePrefix_;  // tiles launched for 1..members members
+    bool smallGroups_ = false;     // split-TF32x3 on tiles of 32 columns (vertical_tf32.cu)
     bool virtualTiles_ = false;    // SIMT tile numbering (GroupTiles::virtualColumns)
     long long imageStride_ = 0;  // tensor-core form: bytes between group images (0: one common image)
     // Tensor-core work units, one table per active member count 1..members.

@@ -129,6 +129,24 @@ cudaError_t launch_grouped_gemm_f64(int R, int S, const double* images, const Gr
                                     ComplexOperand out, const BinBoundary& inBins, const BinBoundary& outBins,
                                     cudaStream_t stream);
 
+// Split-TF32x3 form for small groups (vertical_tf32.cu): FP32 matrices in chunks
+// of kGemmTf32Chunk along s, [chunk][r][s of the chunk], rows zero-padded to a
+// multiple of 8 and 4 more values (36 in full chunks).
+constexpr int kGemmTf32MaxRows = 160;
+constexpr int kGemmTf32Chunk = 32;
+constexpr int gemm_tf32_chunk_row(int left) { return (left < kGemmTf32Chunk ? (left + 7) / 8 * 8 : kGemmTf32Chunk) + 4; }
+constexpr int gemm_tf32_row(int S) {
+    const int full = S / kGemmTf32Chunk;
+    const int left = S - full * kGemmTf32Chunk;
+    return full * gemm_tf32_chunk_row(kGemmTf32Chunk) + (left > 0 ? gemm_tf32_chunk_row(left) : 0);
+}
+// natural [groups][R][S] FP32 -> images [groups][R * gemm_tf32_row(S)] (device).
+cudaError_t gemm_tf32_build_images(const float* natural, long long groups, int R, int S, float* images,
+                                   cudaStream_t stream);
+cudaError_t launch_grouped_gemm_tf32(int R, int S, const float* images, const GroupTiles& tiles, const float2* in,
+                                     float2* out, const BinBoundary& inBins, const BinBoundary& outBins, int* error,
+                                     bool expireWaitForTest, cudaStream_t stream);
+
 // inBins / outBins (optional): cell-addressed operands (BinBoundary) instead of
 // the compact [column][len] arrays.
 cudaError_t launch_grouped_gemm(GemmPrecision p, int R, int S, const void* matrices, const GroupTiles& tiles,
