@@ -734,35 +734,24 @@ __global__ void __launch_bounds__(32 * B, 4) columns_forward_band_warp_kernel(in
 // and no FFT ran at the same speed, and at 16 planes about 1.6x faster).
 // Chunks over the flat index keep every chunk full of real planes except where
 // it crosses a slot's z padding (planes with z >= Nz are skipped).
-// Pass-1 thread (plane b = t % B, butterflies j).  B = 16: the two butterflies
-// of a warp are j and j + 2, and with the 2-mod-16 plane region the pass-1
-// stores and pass-3 loads of a warp fill every bank pair exactly twice.
-// B = 32: a warp is 32 planes of one butterfly, and a plane region of 1 mod 16
-// does the same.
+// Threads (plane b = t % B, butterflies t / B and t / B + 32) do passes 1 and 3, a
+// warp per plane pass 2.  Shared accesses are served half-warp by half-warp: 16 planes
+// of one butterfly, which a plane region of 1 mod 16 puts on 16 bank pairs.  (With 2
+// mod 16 those planes met on 8 of them, and 30 % of the 16-plane inverse's shared
+// wavefronts were repeats: 4059 -> 3955 us for 15 fields of 8 members at Nz 129.)
 // SIGN = +1: inverse (read the band, write every row); SIGN = -1: forward
 // (read every row, write the band times scale).
-template <int B>
-__device__ __forceinline__ int band_wide_butterfly(int t, int q) {
-    if constexpr (B == 16) {
-        const int a = (t >> 5) & 15, c = (t >> 4) & 1;
-        return 4 * (a >> 1) + (a & 1) + 2 * c + 32 * q;
-    } else {
-        return (t >> 5) + 32 * q;
-    }
-}
-template <int B>
-constexpr int band_wide_region() {
-    return B == 16 ? kDirectRegion : 577;  // 577 % 16 == 1, > 511 + 8 * 7
-}
+constexpr int kWideRegion = 577;
+static_assert(kWideRegion % 16 == 1 && kWideRegion > 511 + 8 * 7, "16- and 32-plane region");
 template <int B>
 constexpr size_t band_wide_smem() {
-    return sizeof(float2) * (size_t(B) * band_wide_region<B>() + kDirectTable);
+    return sizeof(float2) * (size_t(B) * kWideRegion + kDirectTable);
 }
 
-// The direct kernels' middle pass with an explicit plane region.
-template <int SIGN, int XP>
+// The direct kernels' middle pass with this plane region.
+template <int SIGN>
 __device__ __forceinline__ void wide_middle_pass(float2* xs, const float2* tt, int warp, int lane) {
-    float2* x = xs + warp * XP;
+    float2* x = xs + warp * kWideRegion;
     float2 v[2][8];
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
@@ -790,7 +779,7 @@ __global__ void __launch_bounds__(32 * B, 32 / B) columns_band_wide_kernel(int n
                                                                           DenseBins bins,
                                                                           const int* __restrict__ bandOf, float scale,
                                                                           const float2* __restrict__ tw) {
-    constexpr int N = kDirectN, XP = band_wide_region<B>();
+    constexpr int N = kDirectN, XP = kWideRegion;
     constexpr int NT = 32 * B;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float2* xs = reinterpret_cast<float2*>(smem_raw);
@@ -807,7 +796,7 @@ __global__ void __launch_bounds__(32 * B, 32 / B) columns_band_wide_kernel(int n
     const long long rowStride = bins.planes * bins.kxStride;
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
-        const int j = band_wide_butterfly<B>(tid, q);
+        const int j = tid / B + 32 * q;
         float2 v[8];
 #pragma unroll
         for (int r = 0; r < 8; ++r) {
@@ -823,13 +812,17 @@ __global__ void __launch_bounds__(32 * B, 32 / B) columns_band_wide_kernel(int n
     __syncthreads();
     {
         const long long pw = p0 + warp;  // planes beyond Nz (or the array) stay idle
-        if (pw < flatPlanes && static_cast<int>(pw % zStride) < nz) wide_middle_pass<SIGN, XP>(xs, tt, warp, lane);
+        if (pw < flatPlanes && static_cast<int>(pw % zStride) < nz) wide_middle_pass<SIGN>(xs, tt, warp, lane);
     }
     __syncthreads();
     if (!inRange) return;
+    // Pass 1's butterflies and rows again, but not its registers: kept across the
+    // middle pass they cost 80 bytes of spills.
+    int tid3 = tid;
+    asm volatile("" : "+r"(tid3));
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
-        const int j = (tid / B) + 32 * q;
+        const int j = tid3 / B + 32 * q;
         const float2* in = xs + b * XP + j;  // pass-3 inputs: elements j + 64 r at j + 72 r
         float2 v[8];
 #pragma unroll
@@ -855,7 +848,7 @@ __global__ void __launch_bounds__(32 * B, 32 / B) columns_band_wide_kernel(int n
 // shared-memory regions alternate between columns; the passes are those of
 // columns_band_wide_kernel.
 constexpr size_t band_pipe_smem() {
-    return sizeof(float2) * (2 * size_t(16) * band_wide_region<16>() + kDirectTable);
+    return sizeof(float2) * (2 * size_t(16) * kWideRegion + kDirectTable);
 }
 template <int SIGN>
 __global__ void __launch_bounds__(512, 1) columns_band_pipe_kernel(int nz, int zStride, long long flatPlanes,
@@ -863,7 +856,7 @@ __global__ void __launch_bounds__(512, 1) columns_band_pipe_kernel(int nz, int z
                                                                    const int* __restrict__ bandOf, float scale,
                                                                    const float2* __restrict__ tw) {
     constexpr int B = 16;
-    constexpr int N = kDirectN, XP = band_wide_region<B>();
+    constexpr int N = kDirectN, XP = kWideRegion;
     constexpr int NT = 32 * B;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float2* xsAll = reinterpret_cast<float2*>(smem_raw);
@@ -884,7 +877,7 @@ __global__ void __launch_bounds__(512, 1) columns_band_pipe_kernel(int nz, int z
         const float2* col = base + bins.planes * kx;
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
-            const int j = band_wide_butterfly<B>(tid, q);
+            const int j = tid / B + 32 * q;
 #pragma unroll
             for (int r = 0; r < 8; ++r) {
                 const int ky = j + 64 * r;
@@ -900,7 +893,7 @@ __global__ void __launch_bounds__(512, 1) columns_band_pipe_kernel(int nz, int z
         float2* xs = xsAll + (i & 1) * B * XP;
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
-            const int j = band_wide_butterfly<B>(tid, q);
+            const int j = tid / B + 32 * q;
             dft8<SIGN>(v[q]);
             float2* o = xs + b * XP + 8 * j + (j >> 1);
 #pragma unroll
@@ -909,7 +902,7 @@ __global__ void __launch_bounds__(512, 1) columns_band_pipe_kernel(int nz, int z
         const int next = kx + static_cast<int>(gridDim.y);
         if (next < columns) load(next, v);
         __syncthreads();
-        if (warpActive) wide_middle_pass<SIGN, XP>(xs, tt, warp, lane);
+        if (warpActive) wide_middle_pass<SIGN>(xs, tt, warp, lane);
         __syncthreads();
         if (inRange) {
             const int band = __ldg(bandOf + kx);

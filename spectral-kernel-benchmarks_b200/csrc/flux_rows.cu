@@ -273,10 +273,23 @@ __global__ void __launch_bounds__(32 * B, 16 / B) rows_flux_kernel(RowFluxArgs a
 // lanes 16-31 plane 2w + 1.
 
 constexpr int kPairM = 256;  // half-length of the 512-point rows
-// Exchange words per plane: one spare per 16 makes the first pass's stride-16
-// stores conflict-free; for 128 and 64 points, whose access phases span two
-// and four planes, the region's length (8 and 4 mod 16) keeps those apart.
-constexpr int pair_xch(int M) { return M + M / 16; }
+// An 8-byte shared access is served half-warp by half-warp, and the 16 lanes of one
+// touch each of the 16 bank pairs once if they are 8 consecutive bins of two adjacent
+// planes (T = M/16 lanes per plane: 16 or 8) or 4 bins of the planes p, p + 1, p + B/2,
+// p + B/2 + 1 (T = 4): so lie the lanes in the TMA forms.  512-point rows with 16 bins
+// of one plane per half-warp, as the cp.async forms' [plane][bin] stages want them,
+// read the swizzled stages with every second access repeated: 5844 -> 5412 us for 8
+// members at Nz 129.
+//
+// Exchange words per plane: one spare per 16 makes the first pass's stride-16 stores
+// conflict-free, and the region's length (8 or 4 mod 16) keeps a half-warp's two or
+// four planes apart.
+constexpr int pair_xch(int M, bool interleaved) { return M + M / 16 + (interleaved ? 8 : 0); }
+// Output tile of the TMA forms, [k][b] like out_slot, for those half-warps.
+template <int B>
+__device__ __forceinline__ int pair_out_slot(int k, int b) {
+    return k * B + (b ^ ((B == 16 ? k & 7 : (k >> 1) & 3) << 1));
+}
 // Bins the pre-processing reads: the 2/3 rule keeps kx < 11 T (T = M/16 lanes
 // per plane; 171 of 176, 86 of 88, 43 of 44), so bins k >= 11 T and, with them,
 // the products of registers m >= 11 (k) and m <= 4 (M - k) are left out.
@@ -300,7 +313,7 @@ constexpr int pair_stage_row() {
 }
 template <int B>
 constexpr size_t pair_smem_words(int keep) {
-    return 2 * size_t(B) * pair_stage_row<B>() + size_t(B) * pair_xch(kPairM) + size_t(keep) * out_row<B>() + kPairM +
+    return 2 * size_t(B) * pair_stage_row<B>() + size_t(B) * pair_xch(kPairM, false) + size_t(keep) * out_row<B>() + kPairM +
            kPairM;
 }
 
@@ -322,7 +335,7 @@ constexpr bool pair_w_in_smem() {
 template <int M, int B, int NS, bool WSM>
 constexpr size_t pair_tma_smem_bytes(int keep) {
     return 1024 + NS * tma_stage_bytes<M, B>() +
-           sizeof(float2) * (size_t(B) * pair_xch(M) + size_t(keep) * out_row<B>() + M + M +
+           sizeof(float2) * (size_t(B) * pair_xch(M, M == kPairM) + size_t(keep) * out_row<B>() + M + M +
                              (WSM ? size_t(M) * B : 0));
 }
 // Byte offset of (kx k, plane b) in a swizzled TMA stage.
@@ -369,6 +382,8 @@ __global__ void __launch_bounds__(M / 16 * B, MINB)
     constexpr int T = M / 16;  // lanes per plane
     constexpr int NT = T * B;
     constexpr int KP = pair_stage_row<B>();
+    constexpr bool PAIRED = TMA && T == 16;  // lanes 2 t and 2 t + 1 hold a warp's two planes
+    constexpr int XCH = pair_xch(M, PAIRED);
     static_assert(M == kPairM || TMA, "the cp.async stages are laid out for 512-point rows");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ __align__(8) unsigned long long stageFull[NST];
@@ -384,7 +399,7 @@ __global__ void __launch_bounds__(M / 16 * B, MINB)
     };
     V* stage0 = stage_of(0);
     V* xchAll = TMA ? reinterpret_cast<V*>(tmaBase + NST * tma_stage_bytes<M, B>()) : stage0 + 2 * B * KP;
-    V* outTile = xchAll + B * pair_xch(M);  // [k][b] at out_slot(k, b)
+    V* outTile = xchAll + B * XCH;          // [k][b] at outSlot(k, b)
     V* tf = outTile + keep * out_row<B>();  // twFull[0..M)
     V* tw2 = tf + M;                     // fft_regs' table: tw2[16 (r - 1) + j] = twHalf[j r]
     // Two-stage TMA forms at 12 warps per SM: W (16 values per thread) lives
@@ -394,8 +409,11 @@ __global__ void __launch_bounds__(M / 16 * B, MINB)
     V* wsm = tw2 + M;
     const int tid = threadIdx.x;
     const int lane = tid & 31;
-    const int t = tid % T;
-    const int pl = tid / T;  // these lanes' plane within the CTA
+    // These lanes' exchange region and plane within the CTA.
+    const int t = PAIRED ? lane >> 1 : tid % T;
+    const int region = PAIRED ? 2 * (tid >> 5) + (lane & 1) : tid / T;
+    const int pl = T == 4 ? (region & 1) | (region & 2) * (B / 4) | (region >> 2) << 1 : region;
+    auto outSlot = [](int k, int b) { return TMA ? pair_out_slot<B>(k, b) : out_slot<B>(k, b); };
     const int zChunks = (a.nz + B - 1) / B;
     const int member = blockIdx.x / zChunks;
     const int z0 = (blockIdx.x % zChunks) * B;
@@ -406,7 +424,7 @@ __global__ void __launch_bounds__(M / 16 * B, MINB)
     V* out = static_cast<V*>(a.binsOut.data);
     const long long inRow = a.binsIn.planes;
     const long long outRow = a.binsOut.planes;
-    PairExchange xch{xchAll + pl * pair_xch(M)};
+    PairExchange xch{xchAll + region * XCH};
 
     for (int i = tid; i < M; i += NT) {
         tf[i] = twFull[i];
@@ -543,7 +561,8 @@ __global__ void __launch_bounds__(M / 16 * B, MINB)
         for (int e = 0; e < 16; ++e) wsm[e * NT + tid] = w[e];
     }
     const float scale = a.scale;
-    const int src = ((T - t) & (T - 1)) + (lane & ~(T - 1));  // lane holding Z[M - k]
+    // Lane holding Z[M - k].
+    const int src = PAIRED ? 2 * ((T - t) & (T - 1)) + (lane & 1) : ((T - t) & (T - 1)) + (lane & ~(T - 1));
     for (int tg = 0; tg < a.targets; ++tg) {
         V acc[16], q[16];
         if (!inverse_row(3 + 3 * tg, q)) return;
@@ -579,13 +598,13 @@ __global__ void __launch_bounds__(M / 16 * B, MINB)
                 const V o = {0.5f * d.y, -0.5f * d.x};
                 X = cadd(ev, cmul(tf[k < M ? k : 0], o));
             }
-            if (k < keep) outTile[out_slot<B>(k, pl)] = X;
+            if (k < keep) outTile[outSlot(k, pl)] = X;
         }
         __syncthreads();
         if (cok) {
             const long long plane = (static_cast<long long>(member) * a.targets + tg) * a.zStride + z0 + cb;
             V* dst = out + plane + outRow * (a.binsOut.kxStride * y + ck);
-            for (int k = ck; k < keep; k += KSTEP, dst += outRow * KSTEP) *dst = outTile[out_slot<B>(k, cb)];
+            for (int k = ck; k < keep; k += KSTEP, dst += outRow * KSTEP) *dst = outTile[outSlot(k, cb)];
         }
         // The next outTile write happens after the next inverse_row's barrier.
     }
