@@ -6,7 +6,6 @@
 #include "autotune.hpp"
 #include "columns_warp.hpp"
 #include "flux_rows.hpp"
-#include "pointwise.hpp"
 
 namespace skb {
 
@@ -71,7 +70,7 @@ FluxPipeline::FluxPipeline(const FluxConfig& cfg) : cfg_(cfg) {
     const std::uint64_t maxPlanes = fused_ ? 1 : 3 * cfg.members * cfg.nz;
     const std::uint64_t binPlanes = fused_ ? cfg.members * cfg.nz * (fieldsIn_ + cfg.targets) : maxPlanes;
     std::uint64_t need = 2 * es * cfg.members * modes_ * cfg.nz * (fieldsIn_ + cfg.targets)  // physIn, physOut
-                         + (fused_ ? 0 : es * volume_ * cfg.members * 7)                   // 3+3+1 volumes
+                         + (fused_ ? 0 : es * volume_ * cfg.members * 7)                   // bound of U, V, W and target bins
                          + 2 * es * cfg.n * (cfg.n / 2 + 1) * binPlanes * 9 / 8;           // bin scratch bound
     size_t freeBytes = 0, totalBytes = 0;
     check_cuda(cudaMemGetInfo(&freeBytes, &totalBytes), "cudaMemGetInfo");
@@ -157,8 +156,7 @@ FluxPipeline::FluxPipeline(const FluxConfig& cfg) : cfg_(cfg) {
         }
     } else {
         shared_.allocate(es * 3 * cfg.members * volume_);
-        deriv_.allocate(es * 3 * cfg.members * volume_);
-        target_.allocate(es * cfg.members * volume_);
+        target_.allocate(horizontal_->blocked_bytes(cfg.members * cfg.nz));
     }
     allocationSeconds = seconds_since(allocStart) + horizontal_->allocationSeconds;
     planningSeconds += horizontal_->planningSeconds;
@@ -166,8 +164,8 @@ FluxPipeline::FluxPipeline(const FluxConfig& cfg) : cfg_(cfg) {
                       cellPhysIn_.bytes() + cellPhysOut_.bytes();
     for (const VerticalPlan* g : gemm_plans()) persistentBytes += g->persistentBytes();
     scratchBytes = horizontal_->scratchBytes + physIn_.bytes() + physOut_.bytes() + shared_.bytes() +
-                   deriv_.bytes() + target_.bytes() + binsIn_.bytes() + binsOut_.bytes();
-    // Staged: 2 GEMMs, 2 launches per inverse / forward horizontal, members pointwise per target.
+                   target_.bytes() + binsIn_.bytes() + binsOut_.bytes();
+    // Staged: 2 GEMMs, columns and rows of U, V, W, then columns, row product and columns per target.
     // Fused: GEMM, embed+columns, fused rows, columns+retention, GEMM.  With
     // operator families each GEMM is one launch per family.
     if (fused_ && dense_ && cfg.n == 512) {
@@ -184,7 +182,7 @@ FluxPipeline::FluxPipeline(const FluxConfig& cfg) : cfg_(cfg) {
         const std::uint64_t inChunks = cfg.members * fieldsIn_ * zStride_ / 16;
         horizontal_->set_band_forms(inChunks >= 127 ? kBand16Pipe16 : kBand16, kBandRegs);
     }
-    launches_ = (fused_ ? 5 : 2 + 2 + cfg.targets * (2 + cfg.members + 2)) + (families_ ? 2 : 0);
+    launches_ = (fused_ ? 5 : 2 + 2 + cfg.targets * 3) + (families_ ? 2 : 0);
     apply_tuned(nullptr, nullptr, nullptr, nullptr);
 }
 
@@ -192,8 +190,7 @@ FluxPipeline::FluxPipeline(const FluxConfig& cfg) : cfg_(cfg) {
 //   work-unit size (M-tiles per unit) of each tensor-core GEMM, 4 / 8 / 16 / 32;
 //   the 512-point row kernel's form (one plane per warp, or two planes per
 //   warp with the 16 x 16 FFT) and its z-planes per CTA, 4 / 8 / 16;
-//   kernel form of each 512-point band column stage, direct / warp-per-plane /
-//   persistent direct.
+//   kernel form of each 512-point band column stage (columns_warp.hpp).
 // With buffers, missing choices are measured on them (tune_pick); without,
 // only cached choices are applied.  Returns the choices in force.
 std::vector<TuneEntry> FluxPipeline::apply_tuned(const void* modalIn, void* modalOut, cudaStream_t s,
@@ -498,33 +495,25 @@ void FluxPipeline::run(const void* modalIn, void* modalOut, cudaStream_t s, Reco
         return v;
     };
     const double triplePlanes = 3.0 * M * nz;
-    auto inverseTriple = [&](std::uint64_t firstField, void* real) {
-        const ViewSet v = triple(firstField);
-        horizontal_->inverse_columns(v, s);
+    auto inverseColumns = [&](std::uint64_t firstField) {
+        horizontal_->inverse_columns(triple(firstField), s);
         if (rec) rec->end("columns_inverse_embed", 1, triplePlanes * (compactPlane + binsPlane), 0.0);
-        horizontal_->inverse_rows(real, 3 * M * nz, s);
-        if (rec) rec->end("rows_inverse_c2r", 1, triplePlanes * (binsPlane + realPlane), 0.0);
     };
-    inverseTriple(0, shared_.get());
+    inverseColumns(0);
+    horizontal_->inverse_rows(shared_.get(), 3 * M * nz, s);
+    if (rec) rec->end("rows_inverse_c2r", 1, triplePlanes * (binsPlane + realPlane), 0.0);
     const double scale = 1.0 / (n * n * n * n);
-    const int sms = sm_count();
     for (std::uint64_t t = 0; t < T; ++t) {
-        inverseTriple(3 + 3 * t, deriv_.get());
-        for (std::uint64_t m = 0; m < M; ++m) {
-            check_cuda(launch_pointwise(f64(), static_cast<long long>(volume_), scale,
-                                        shared_.get<unsigned char>() + es * 3 * m * volume_,
-                                        deriv_.get<unsigned char>() + es * 3 * m * volume_,
-                                        target_.get<unsigned char>() + es * m * volume_, sms, s),
-                       "pointwise advection kernel");
-        }
-        if (rec) rec->end("pointwise", M, 7.0 * es * double(volume_) * M, 6.0 * double(volume_) * M);
+        inverseColumns(3 + 3 * t);
+        horizontal_->product_rows(shared_.get(), M, scale, target_.get(), s);
+        if (rec)
+            rec->end("rows_product", 1, triplePlanes * (binsPlane + realPlane) + double(M) * nz * binsPlane,
+                     6.0 * double(volume_) * M);
         ViewSet out{};
         out.count = static_cast<int>(M);
         for (std::uint64_t m = 0; m < M; ++m)
             out.v[m] = {physOut + ces * ((m * H * T + t) * nz), nullptr, static_cast<long long>(T * nz)};
-        horizontal_->forward_rows(target_.get(), M * nz, s);
-        if (rec) rec->end("rows_forward_r2c", 1, double(M) * nz * (realPlane + binsPlane), 0.0);
-        horizontal_->forward_columns(out, 1.0, s);
+        horizontal_->forward_columns(target_.get(), out, 1.0, s);
         if (rec) rec->end("columns_forward_gather", 1, double(M) * nz * (binsPlane + compactPlane), 0.0);
     }
     gemm_forward(modalOut, s, M, false);

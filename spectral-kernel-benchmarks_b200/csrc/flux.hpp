@@ -100,7 +100,7 @@ private:
     std::uint64_t modes_ = 0, nj_ = 0, fieldsIn_ = 0, volume_ = 0;
     std::unique_ptr<HorizontalPlan> horizontal_;
     std::unique_ptr<VerticalPlan> inverseGemm_, forwardGemm_;
-    DeviceBuffer physIn_, shared_, deriv_, target_, physOut_;
+    DeviceBuffer physIn_, shared_, target_, physOut_;
     // Fused split-precision path: column-transformed bins of every input slot
     // and of every target.
     bool fused_ = false;

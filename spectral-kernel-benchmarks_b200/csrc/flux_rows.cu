@@ -1,8 +1,8 @@
 // Fused row stage of the split-precision flux (FP32).
 //
 // One CTA owns one row y of B consecutive z-planes of one ensemble member and
-// does, entirely on chip, what the staged path spreads over three kernels and
-// seven real volumes (benchmark.cpp:4405-4424 order):
+// does, entirely on chip, what the staged path spreads over a row kernel for U, V and
+// W and one per target, with three real volumes (benchmark.cpp:4405-4424 order):
 //   U,V,W rows      <- c2r of the column-transformed bins of input slots 0..2,
 //                      kept in registers;
 //   for each target t:
@@ -11,7 +11,10 @@
 //     target bins    <- r2c of the target row, kx < keep.
 // The c2r / r2c are the same half-length complex FFT formulation as the
 // staged row kernels (horizontal.cu), so both paths share their numerics.
-// Each warp owns one z-plane and transforms it with warp-synchronous passes
+// Two kernels: 128-, 256- and 512-point rows run several planes per warp
+// (rows_flux_pair_kernel, below); in the other, for 64-point rows and as a choice of
+// the autotuner at 512 points, each warp owns one z-plane and transforms it with
+// warp-synchronous passes
 // (warp_fft; for 512-point rows warp_fft_rr, whose first and last passes work
 // in registers); every lane keeps the same Nx/64 x-pairs of its plane across
 // all transforms, which is what lets U,V,W and the product stay in registers.
@@ -260,7 +263,8 @@ __global__ void __launch_bounds__(32 * B, 16 / B) rows_flux_kernel(RowFluxArgs a
 }
 
 // ---------------------------------------------------------------------------
-// 512-point rows, two planes per warp.
+// 512-point rows, two planes per warp, and 256- and 128-point rows with four and
+// eight (T = 8 and 4 lanes per plane, the second radix 8 and 4).
 //
 // The 256-point complex FFT of the half-length formulation is split 16 x 16:
 // lane t of a half-warp holds elements t + 16 m (m = 0..15) of its plane's
@@ -269,8 +273,7 @@ __global__ void __launch_bounds__(32 * B, 16 / B) rows_flux_kernel(RowFluxArgs a
 // registers leave output k = t + 16 k1 in register k1 — the same lane-owned
 // positions as the input, so U, V, W and the product stay in registers across
 // all transforms as in the warp-per-plane kernel, with one shared-memory
-// exchange per transform instead of two.  Lanes 0-15 own plane 2w of warp w,
-// lanes 16-31 plane 2w + 1.
+// exchange per transform instead of two.  Warp w owns planes 2w and 2w + 1.
 
 constexpr int kPairM = 256;  // half-length of the 512-point rows
 // An 8-byte shared access is served half-warp by half-warp, and the 16 lanes of one

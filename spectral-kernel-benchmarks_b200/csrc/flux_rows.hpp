@@ -17,8 +17,9 @@ struct RowFluxArgs {
     const void* twHalf;   // exp(-2 pi i k/(nx/2)), float2
     const void* twFull;   // exp(-2 pi i k/nx), float2
     int planes = 8;       // z-planes per CTA: 4, 8 or 16, and 24 for the two-planes-per-warp form (an autotuner choice)
-    // Nx = 512 only: two planes per warp (16 lanes each, 16 x-pairs per lane)
-    // with a radix-16 x radix-16 FFT; needs planes 8 or 16 (autotuner choice).
+    // Nx = 512 (128 and 256 always run several planes per warp): two planes per warp (16
+    // lanes each, 16 x-pairs per lane) with a radix-16 x radix-16 FFT; needs planes 8 or
+    // 16 (autotuner choice).
     // 2: the 8-plane form compiled for three resident CTAs per SM.
     int pairs = 0;
     // Two-planes-per-warp forms only: 1 fills each slot's stage with one TMA

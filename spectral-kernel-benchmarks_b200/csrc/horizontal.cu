@@ -103,42 +103,24 @@ __device__ __forceinline__ int pair_source(int j) {
 // z[m] = x[2m] + i x[2m+1], transformed, then split into the real spectrum:
 //   X[k] = s + W^k o,  X[M-k] = conj(s - W^k o),  W = e^{-2 pi i/NX},
 //   s = (Z[k] + conj Z[M-k])/2,  o = -i (Z[k] - conj Z[M-k])/2.
+//
+// row_forward: v holds the row side's elements; out is bin 0 of the plane side's
+// plane (bins `stride` apart), written where live.
 template <typename T, int M>
-__global__ void __launch_bounds__(RowShape<T, M>::NT, RowShape<T, M>::kCtas)
-    rows_forward_kernel(int ny, long long planes, int keep, const T* __restrict__ real, DenseBins bins,
-                        const cx<T>* __restrict__ tw, const cx<T>* __restrict__ twFull) {
+__device__ __forceinline__ void row_forward(cx<T> (&v)[RowShape<T, M>::E], cx<T>* data, cx<T>* out, long long stride,
+                                            bool live, int keep, const cx<T>* __restrict__ tw,
+                                            const cx<T>* __restrict__ twFull) {
     using V = cx<T>;
     using S = RowShape<T, M>;
-    constexpr int NX = 2 * M, R = S::R, Ns = S::Ns;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    V* data = reinterpret_cast<V*>(smem_raw);
+    constexpr int R = S::R, Ns = S::Ns;
     const int tid = threadIdx.x;
-    const long long p0 = (long long)blockIdx.x * S::B;
-    const int y = blockIdx.y;
-    V v[S::E];
-    grid_wait();
-    {
-        const int t = tid % S::TPR;
-        const int b = tid / S::TPR;
-        if (p0 + b < planes) {
-            const V* row = reinterpret_cast<const V*>(real + ((p0 + b) * ny + y) * NX) + t;
-#pragma unroll
-            for (int e = 0; e < S::E; ++e) v[e] = row[S::TPR * e];
-        } else {
-#pragma unroll
-            for (int e = 0; e < S::E; ++e) v[e] = {T(0), T(0)};
-        }
-        if constexpr (S::TPR > 1) {
-            RowExchange<S> xch{data, b};
-            fft_regs_head<T, M, S::E, -1, Ns>(v, t, tw, xch);
-            __syncthreads();
-        }
+    if constexpr (S::TPR > 1) {
+        RowExchange<S> xch{data, tid / S::TPR};
+        fft_regs_head<T, M, S::E, -1, Ns>(v, tid % S::TPR, tw, xch);
+        __syncthreads();
     }
     const int b = tid % S::B;
     const int g = tid / S::B;
-    const bool live = p0 + b < planes;
-    const long long stride = bins.planes;
-    V* out = reinterpret_cast<V*>(bins.data) + bins.offset(live ? p0 + b : 0) + stride * bins.kxStride * y;
     auto split = [&](int k, V zk, V zmk) {
         const V zm = cconj(zmk);
         const V s = cscale(cadd(zk, zm), T(0.5));
@@ -211,27 +193,21 @@ __global__ void __launch_bounds__(RowShape<T, M>::NT, RowShape<T, M>::kCtas)
 // s = X[k] + conj X[M-k], t = e^{+2 pi i k/NX} (X[k] - conj X[M-k]), then an
 // inverse length-M FFT gives x[2m] + i x[2m+1].  The radices run in the
 // forward kernel's order reversed, so the plane side has the same butterflies.
-template <typename T, int M>
-__global__ void __launch_bounds__(RowShape<T, M>::NT, RowShape<T, M>::kCtas)
-    rows_inverse_kernel(int ny, long long planes, int keep, DenseBins bins, T* __restrict__ real,
-                        const cx<T>* __restrict__ tw, const cx<T>* __restrict__ twFull) {
+//
+// row_inverse: in is bin 0 of the plane side's plane (bins `stride` apart), read
+// where live; leaves the row side's elements in v.  `between` runs between the two
+// sides (loads to have in flight during the row side's passes).
+template <typename T, int M, typename F>
+__device__ __forceinline__ void row_inverse(cx<T> (&v)[RowShape<T, M>::E], cx<T>* data, const cx<T>* in,
+                                            long long stride, bool live, int keep, const cx<T>* __restrict__ tw,
+                                            const cx<T>* __restrict__ twFull, F between) {
     using V = cx<T>;
     using S = RowShape<T, M>;
-    constexpr int NX = 2 * M, R = S::R, Ns = S::Ns;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    V* data = reinterpret_cast<V*>(smem_raw);
+    constexpr int R = S::R, Ns = S::Ns;
     const int tid = threadIdx.x;
-    const long long p0 = (long long)blockIdx.x * S::B;
-    const int y = blockIdx.y;
-    V v[S::E];
-    grid_wait();
     {
         const int b = tid % S::B;
         const int g = tid / S::B;
-        const bool live = p0 + b < planes;
-        const long long stride = bins.planes;
-        const V* in =
-            reinterpret_cast<const V*>(bins.data) + bins.offset(live ? p0 + b : 0) + stride * bins.kxStride * y;
         auto load = [&](int k) -> V { return live && k < keep ? in[stride * k] : V{T(0), T(0)}; };
         // (X[k], X[M-k]) -> (Z[k], Z[M-k])
         auto merge = [&](int k, V& xk, V& xm) {
@@ -321,19 +297,151 @@ __global__ void __launch_bounds__(RowShape<T, M>::NT, RowShape<T, M>::kCtas)
             }
         }
     }
-    const int t = tid % S::TPR;
-    const int b = tid / S::TPR;
+    between();
     if constexpr (S::TPR > 1) {
+        const int t = tid % S::TPR;
         __syncthreads();
-        RowExchange<S> xch{data, b};
+        RowExchange<S> xch{data, tid / S::TPR};
 #pragma unroll
         for (int e = 0; e < S::E; ++e) v[e] = xch.load(t + S::TPR * e);
         fft_regs<T, M, S::E, +1, R>(v, t, tw, xch);
     }
-    if (p0 + b >= planes) return;
-    V* row = reinterpret_cast<V*>(real + ((p0 + b) * ny + y) * NX) + t;
+}
+
+// Grid (plane chunks, ny).
+template <typename T, int M>
+__global__ void __launch_bounds__(RowShape<T, M>::NT, RowShape<T, M>::kCtas)
+    rows_forward_kernel(int ny, long long planes, int keep, const T* __restrict__ real, DenseBins bins,
+                        const cx<T>* __restrict__ tw, const cx<T>* __restrict__ twFull) {
+    using V = cx<T>;
+    using S = RowShape<T, M>;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const long long p0 = (long long)blockIdx.x * S::B;
+    const int y = blockIdx.y;
+    V v[S::E];
+    grid_wait();
+    const long long row = p0 + threadIdx.x / S::TPR;
+    if (row < planes) {
+        const V* from = reinterpret_cast<const V*>(real + (row * ny + y) * (2 * M)) + threadIdx.x % S::TPR;
 #pragma unroll
-    for (int e = 0; e < S::E; ++e) row[S::TPR * e] = v[e];
+        for (int e = 0; e < S::E; ++e) v[e] = from[S::TPR * e];
+    } else {
+#pragma unroll
+        for (int e = 0; e < S::E; ++e) v[e] = {T(0), T(0)};
+    }
+    const long long p = p0 + threadIdx.x % S::B;
+    const bool live = p < planes;
+    V* out = reinterpret_cast<V*>(bins.data) + bins.offset(live ? p : 0) + bins.planes * bins.kxStride * y;
+    row_forward<T, M>(v, reinterpret_cast<V*>(smem_raw), out, bins.planes, live, keep, tw, twFull);
+}
+
+template <typename T, int M>
+__global__ void __launch_bounds__(RowShape<T, M>::NT, RowShape<T, M>::kCtas)
+    rows_inverse_kernel(int ny, long long planes, int keep, DenseBins bins, T* __restrict__ real,
+                        const cx<T>* __restrict__ tw, const cx<T>* __restrict__ twFull) {
+    using V = cx<T>;
+    using S = RowShape<T, M>;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const long long p0 = (long long)blockIdx.x * S::B;
+    const int y = blockIdx.y;
+    V v[S::E];
+    grid_wait();
+    const long long p = p0 + threadIdx.x % S::B;
+    const bool live = p < planes;
+    const V* in = reinterpret_cast<const V*>(bins.data) + bins.offset(live ? p : 0) + bins.planes * bins.kxStride * y;
+    row_inverse<T, M>(v, reinterpret_cast<V*>(smem_raw), in, bins.planes, live, keep, tw, twFull, [] {});
+    const long long row = p0 + threadIdx.x / S::TPR;
+    if (row >= planes) return;
+    V* to = reinterpret_cast<V*>(real + (row * ny + y) * (2 * M)) + threadIdx.x % S::TPR;
+#pragma unroll
+    for (int e = 0; e < S::E; ++e) to[S::TPR * e] = v[e];
+}
+
+// One target of the staged flux, for B planes (member m, level z) of one y: the rows
+// of the three derivative slots are transformed one after the other and multiplied,
+// in registers, by the rows of U, V and W; the negated, scaled sum goes back through
+// the forward transform to the target's bins:
+//   bins(m, z) <- r2c(-scale (u q_x + v q_y + w q_z)),  q_f = c2r(bins(3 m + f, z)).
+// Neither the derivatives' real rows nor the product's are stored: 8 of the 11 real
+// volumes that inverse rows, pointwise product and forward rows moved per target.
+// Bound: latency, at two CTAs of 128 threads per SM (FP64, 255 registers: the sum, a
+// slot's row and the velocity row in flight), 3.6 TB/s.  Row stages of a flux, before
+// and now: FP64 512^2, Nz 129, 4 targets 2869 -> 2005 us, 256^2, Nz 65, 3 targets of 2
+// members 597 -> 390; FP32 512^2, Nz 65 842 -> 686, 256^2 337 -> 225; FP64 1024^2, Nz
+// 17 1324 -> 1235, FP32 836 -> 877 (1141 with every pass of the rows in shared
+// memory).  512^2 without the L2 prefetches 2400, with 168 registers for a third CTA
+// (spills) 2037-2051.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
+template <typename T, int M>
+struct ProductShape {
+    using S = RowShape<T, M>;
+    static constexpr int regs = sizeof(T) == 8 ? (S::E > 8 ? 255 : 128) : (S::E > 8 ? 128 : 80);
+    static constexpr int bySmem = int(size_t(227 * 1024) / (S::kBytes + 1024));
+    static constexpr int byRegs = 65536 / (S::NT * regs);
+    static constexpr int least = bySmem < byRegs ? bySmem : byRegs;
+    static constexpr int kCtas = least < 1 ? 1 : least > 16 ? 16 : least;
+};
+
+template <typename T, int M>
+__global__ void __launch_bounds__(RowShape<T, M>::NT, ProductShape<T, M>::kCtas)
+    rows_product_kernel(int ny, int nz, long long planes, int keep, T scale, const T* __restrict__ velocity,
+                        DenseBins in, DenseBins bins, const cx<T>* __restrict__ twInverse,
+                        const cx<T>* __restrict__ twForward, const cx<T>* __restrict__ twFull) {
+    using V = cx<T>;
+    using S = RowShape<T, M>;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    V* data = reinterpret_cast<V*>(smem_raw);
+    const long long p0 = (long long)blockIdx.x * S::B;
+    const int y = blockIdx.y;
+    // Plane side: this thread's target plane and slot 0's plane of it.
+    const long long p = p0 + threadIdx.x % S::B;
+    const bool live = p < planes;
+    const long long first = live ? p + p / nz * 2 * nz : 0;
+    // Row side: its row of U.
+    const long long row = p0 + threadIdx.x / S::TPR;
+    const bool rowLive = row < planes;
+    const long long volume = (long long)nz * ny * M;  // complex pairs of one slot
+    const V* vel = reinterpret_cast<const V*>(velocity) +
+                   (rowLive ? ((row + row / nz * 2 * nz) * ny + y) * M : 0) + threadIdx.x % S::TPR;
+    grid_wait();
+    V sum[S::E];
+#pragma unroll
+    for (int e = 0; e < S::E; ++e) sum[e] = {T(0), T(0)};
+    auto bins_of = [&](int f) {
+        return reinterpret_cast<const V*>(in.data) + in.offset(first + (long long)f * nz) +
+               in.planes * in.kxStride * y;
+    };
+#pragma unroll 1
+    for (int f = 0; f < 3; ++f) {
+        V v[S::E];
+        const V* from = bins_of(f);
+        if (f > 0) __syncthreads();  // the previous slot's exchange has been read
+        // L2 prefetches, a 128-byte line each: this slot's velocity rows and, by the
+        // first and last plane's threads, the next slot's bins.
+        constexpr int kLine = phase_lanes<T>();
+        if (rowLive)
+            for (int e = int(threadIdx.x % S::TPR) * kLine; e < M; e += S::TPR * kLine)
+                prefetch_l2(vel + f * volume + e - int(threadIdx.x % S::TPR));
+        if (f < 2 && live && (threadIdx.x % S::B == 0 || threadIdx.x % S::B == S::B - 1)) {
+            const V* next = bins_of(f + 1);
+            for (int k = threadIdx.x / S::B; k < keep; k += S::TPR) prefetch_l2(next + in.planes * k);
+        }
+        V u[S::E];
+        row_inverse<T, M>(v, data, from, in.planes, live, keep, twInverse, twFull, [&] {
+#pragma unroll
+            for (int e = 0; e < S::E; ++e) u[e] = rowLive ? __ldg(vel + f * volume + S::TPR * e) : V{T(0), T(0)};
+        });
+#pragma unroll
+        for (int e = 0; e < S::E; ++e)
+            sum[e] = f == 0 ? V{u[e].x * v[e].x, u[e].y * v[e].y}
+                            : V{sum[e].x + u[e].x * v[e].x, sum[e].y + u[e].y * v[e].y};
+    }
+#pragma unroll
+    for (int e = 0; e < S::E; ++e) sum[e] = {-scale * sum[e].x, -scale * sum[e].y};
+    __syncthreads();
+    V* out = reinterpret_cast<V*>(bins.data) + bins.offset(live ? p : 0) + bins.planes * bins.kxStride * y;
+    row_forward<T, M>(sum, data, out, bins.planes, live, keep, twForward, twFull);
 }
 
 // Length-1 rows (Nx = 2): X[0] = x0 + x1, X[1] = x0 - x1.
@@ -356,6 +464,30 @@ __global__ void rows_pair_kernel(int dir, int ny, long long planes, int keep, co
         realOut[(p * ny + y) * 2] = a + c;
         realOut[(p * ny + y) * 2 + 1] = a - c;
     }
+}
+
+// The product stage for such rows.
+template <typename T>
+__global__ void rows_product_pair_kernel(int ny, int nz, long long planes, int keep, T scale,
+                                         const T* __restrict__ velocity, DenseBins in, DenseBins bins) {
+    using V = cx<T>;
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= planes * ny) return;
+    const long long p = i % planes;
+    const long long y = i / planes;
+    T s0 = T(0), s1 = T(0);
+    for (int f = 0; f < 3; ++f) {
+        const long long slot = p + p / nz * 2 * nz + (long long)f * nz;
+        const V* b = reinterpret_cast<const V*>(in.data) + in.offset(slot) + in.planes * in.kxStride * y;
+        const T a = b[0].x;
+        const T c = keep > 1 ? b[in.planes].x : T(0);
+        const T* u = velocity + (slot * ny + y) * 2;
+        s0 += u[0] * (a + c);
+        s1 += u[1] * (a - c);
+    }
+    V* b = reinterpret_cast<V*>(bins.data) + bins.offset(p) + bins.planes * bins.kxStride * y;
+    b[0] = {-scale * s0 - scale * s1, T(0)};
+    if (keep > 1) b[bins.planes] = {-scale * s0 + scale * s1, T(0)};
 }
 
 // ---------------------------------------------------------------------------
@@ -584,6 +716,29 @@ cudaError_t rows_inverse_t(int nx, int ny, long long planes, int keep, DenseBins
     return cudaGetLastError();
 }
 
+template <typename T>
+cudaError_t rows_product_t(int nx, int ny, int nz, long long planes, int keep, double scale, const void* velocity,
+                           DenseBins in, DenseBins out, const void* twInverse, const void* twForward,
+                           const void* twFull, cudaStream_t stream) {
+    if (nx == 2) {
+        const long long n = planes * ny;
+        rows_product_pair_kernel<T><<<unsigned((n + 255) / 256), 256, 0, stream>>>(
+            ny, nz, planes, keep, T(scale), static_cast<const T*>(velocity), in, out);
+        return cudaGetLastError();
+    }
+    SKB_HALF_SWITCH(nx / 2, {
+        using S = RowShape<T, L>;
+        auto kernel = rows_product_kernel<T, L>;
+        const cudaError_t err = allow_smem(kernel, S::kBytes);
+        if (err != cudaSuccess) return err;
+        const dim3 grid(unsigned((planes + S::B - 1) / S::B), unsigned(ny));
+        return launch_chained(kernel, grid, S::NT, S::kBytes, stream, ny, nz, planes, keep, T(scale),
+                              static_cast<const T*>(velocity), in, out, static_cast<const cx<T>*>(twInverse),
+                              static_cast<const cx<T>*>(twForward), static_cast<const cx<T>*>(twFull));
+    });
+    return cudaGetLastError();
+}
+
 template <typename T, int SIGN, ColumnIo IN, ColumnIo OUT>
 cudaError_t columns_t(int ny, int columns, long long planes, DenseBins in, DenseBins out, int nz, const ViewSet& views,
                       const int* cells, double scale, const void* tw, cudaStream_t stream) {
@@ -617,6 +772,17 @@ cudaError_t launch_rows_inverse(Precision p, int nx, int ny, long long planes, i
     if (planes <= 0) return cudaSuccess;
     return p == Precision::f64 ? rows_inverse_t<double>(nx, ny, planes, keep, bins, real, twHalf, twFull, stream)
                                : rows_inverse_t<float>(nx, ny, planes, keep, bins, real, twHalf, twFull, stream);
+}
+
+cudaError_t launch_rows_product(Precision p, int nx, int ny, int nz, int members, int keep, double scale,
+                                const void* velocity, DenseBins in, DenseBins out, const void* twInverse,
+                                const void* twForward, const void* twFull, cudaStream_t stream) {
+    const long long planes = (long long)members * nz;
+    if (planes <= 0) return cudaSuccess;
+    return p == Precision::f64 ? rows_product_t<double>(nx, ny, nz, planes, keep, scale, velocity, in, out, twInverse,
+                                                        twForward, twFull, stream)
+                               : rows_product_t<float>(nx, ny, nz, planes, keep, scale, velocity, in, out, twInverse,
+                                                       twForward, twFull, stream);
 }
 
 cudaError_t launch_columns_dense(Precision p, int sign, int ny, int columns, long long planes, DenseBins in,

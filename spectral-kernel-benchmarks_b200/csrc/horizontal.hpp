@@ -111,6 +111,13 @@ cudaError_t launch_rows_forward(Precision p, int nx, int ny, long long planes, i
                                 DenseBins bins, const void* twHalf, const void* twFull, cudaStream_t stream);
 cudaError_t launch_rows_inverse(Precision p, int nx, int ny, long long planes, int keep, DenseBins bins, void* real,
                                 const void* twHalf, const void* twFull, cudaStream_t stream);
+// One target of the flux: `in` holds the bins of three derivative slots of
+// every member (slot 3 m + f, nz planes each), `velocity` the real volumes of U, V and
+// W in the same slot order; `out` gets the bins of -scale (u q_x + v q_y + w q_z), nz
+// planes per member.
+cudaError_t launch_rows_product(Precision p, int nx, int ny, int nz, int members, int keep, double scale,
+                                const void* velocity, DenseBins in, DenseBins out, const void* twInverse,
+                                const void* twForward, const void* twFull, cudaStream_t stream);
 
 // y-direction transforms over kx in [0, columns).
 // sign = -1 forward, +1 inverse.

@@ -107,8 +107,7 @@ HorizontalPlan::HorizontalPlan(const Workload& w, Precision p, bool pruned, std:
     modeKx_ = upload_vector(tables.modeKx);
     modeKy_ = upload_vector(tables.modeKy);
     modeConj_ = upload_vector(tables.modeConj);
-    const size_t binBytes = static_cast<size_t>(w.ny) * keep_ * (scratch_blocks(maxPlanes) << kScratchShift) * 2 * element_bytes(p);
-    bins_.allocate(binBytes);
+    bins_.allocate(blocked_bytes(maxPlanes));
     {
         // Per-column band of the retained cells, and whether it is exact.
         std::vector<int> band(static_cast<size_t>(keep_), -1);
@@ -148,11 +147,24 @@ void HorizontalPlan::forward_rows(const void* real, std::uint64_t planes, cudaSt
 }
 
 void HorizontalPlan::forward_columns(const ViewSet& views, double scale, cudaStream_t s) const {
-    const auto planes = static_cast<std::uint64_t>(views.count) * w_.nz;
-    if (planes > maxPlanes_) throw Error(-1, "plane count exceeds the plan's scratch");
-    check_cuda(launch_columns_gather(p_, static_cast<int>(w_.ny), static_cast<int>(w_.nz), keep_, scratch(planes),
-                                     views, tables(), scale, colTable_.get(), s),
+    if (static_cast<std::uint64_t>(views.count) * w_.nz > maxPlanes_)
+        throw Error(-1, "plane count exceeds the plan's scratch");
+    forward_columns(bins_.get(), views, scale, s);
+}
+
+void HorizontalPlan::forward_columns(const void* target, const ViewSet& views, double scale, cudaStream_t s) const {
+    check_cuda(launch_columns_gather(p_, static_cast<int>(w_.ny), static_cast<int>(w_.nz), keep_,
+                                     blocked(const_cast<void*>(target)), views, tables(), scale, colTable_.get(), s),
                "column c2c + retention kernel");
+}
+
+void HorizontalPlan::product_rows(const void* velocity, std::uint64_t members, double scale, void* target,
+                                  cudaStream_t s) const {
+    if (3 * members * w_.nz > maxPlanes_) throw Error(-1, "plane count exceeds the plan's scratch");
+    check_cuda(launch_rows_product(p_, static_cast<int>(w_.nx), static_cast<int>(w_.ny), static_cast<int>(w_.nz),
+                                   static_cast<int>(members), keep_, scale, velocity, blocked(bins_.get()),
+                                   blocked(target), rowInverse_.get(), rowForward_.get(), twFull_.get(), s),
+               "row product kernel");
 }
 
 void HorizontalPlan::inverse_columns(const ViewSet& views, cudaStream_t s) const {

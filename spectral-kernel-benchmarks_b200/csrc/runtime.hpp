@@ -105,9 +105,14 @@ public:
     std::uint64_t scratch_blocks(std::uint64_t planes) const {
         return (planes + (std::uint64_t(1) << kScratchShift) - 1) >> kScratchShift;
     }
-    DenseBins scratch(std::uint64_t) const {
+    DenseBins scratch(std::uint64_t) const { return blocked(bins_.get()); }
+    std::uint64_t blocked_bytes(std::uint64_t planes) const {
+        return w_.ny * static_cast<std::uint64_t>(keep_) * (scratch_blocks(planes) << kScratchShift) * 2 *
+               element_bytes(p_);
+    }
+    DenseBins blocked(void* data) const {
         const long long block = 1LL << kScratchShift;
-        return {bins_.get(), block, static_cast<long long>(keep_), kScratchShift,
+        return {data, block, static_cast<long long>(keep_), kScratchShift,
                 block * static_cast<long long>(keep_) * static_cast<long long>(w_.ny)};
     }
 
@@ -118,6 +123,10 @@ public:
     void forward_columns(const ViewSet& views, double scale, cudaStream_t s) const;
     void inverse_columns(const ViewSet& views, cudaStream_t s) const;
     void inverse_rows(void* real, std::uint64_t planes, cudaStream_t s) const;
+    // Flux target of the derivative slots in the scratch (launch_rows_product), and
+    // its column stage; `target` holds blocked_bytes(members * Nz) bytes.
+    void product_rows(const void* velocity, std::uint64_t members, double scale, void* target, cudaStream_t s) const;
+    void forward_columns(const void* target, const ViewSet& views, double scale, cudaStream_t s) const;
     // Full-grid dense forms (keep = Nx/2+1): WVM spectrum with `planes` planes.
     void forward_dense(const void* real, void* wvm, std::uint64_t planes, cudaStream_t s) const;
     void inverse_dense(const void* wvm, void* real, std::uint64_t planes, cudaStream_t s) const;
