@@ -133,17 +133,19 @@ __global__ void __launch_bounds__(kThreads, resident<MH>())
         const double* src = image + static_cast<long long>(c) * kChunk * R;
         double* sA = stageA(b);
         for (int i = tid; i < R * gemm_f64_chunk_row(left) / 2; i += kThreads) copy16(sA + 2 * i, src + 2 * i);
-        double* sX = stageX(b);
-        for (int i = tid; i < ncols * kChunk; i += kThreads) {
-            const int col = i / kChunk, s = i % kChunk;
-            if (s >= steps) continue;
-            const bool ok = s < left;
-            const long long at = ok ? colIn[col] + c * kChunk + s : 0;
-            if (split) {
-                copy_or_zero<8>(sX + 2 * i, static_cast<const double*>(in.re) + at, ok);
-                copy_or_zero<8>(sX + 2 * i + 1, static_cast<const double*>(in.im) + at, ok);
-            } else {
-                copy_or_zero<16>(sX + 2 * i, static_cast<const double2*>(in.re) + at, ok);
+        // Warp w copies columns w + 8 k, a lane one step of the chunk.
+        if (lane < steps) {
+            const bool ok = lane < left;
+            const int first = c * kChunk + lane;
+            double* sX = stageX(b) + 2 * (warp * kChunk + lane);
+            for (int col = warp; col < ncols; col += kThreads / 32, sX += 2 * kChunk * (kThreads / 32)) {
+                const long long at = ok ? colIn[col] + first : 0;
+                if (split) {
+                    copy_or_zero<8>(sX, static_cast<const double*>(in.re) + at, ok);
+                    copy_or_zero<8>(sX + 1, static_cast<const double*>(in.im) + at, ok);
+                } else {
+                    copy_or_zero<16>(sX, static_cast<const double2*>(in.re) + at, ok);
+                }
             }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
