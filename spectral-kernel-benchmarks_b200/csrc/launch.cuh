@@ -36,7 +36,11 @@ cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, unsigned threads, si
     config.stream = stream;
     config.attrs = &attribute;
     config.numAttrs = 1;
-    return cudaLaunchKernelEx(&config, kernel, static_cast<P>(args)...);
+    // A refused launch is reported here, once: the code left standing would be the
+    // next cudaGetLastError()'s, in a later launch or in the caller's own code.
+    const cudaError_t err = cudaLaunchKernelEx(&config, kernel, static_cast<P>(args)...);
+    if (err != cudaSuccess) cudaGetLastError();
+    return err;
 }
 
 }  // namespace skb

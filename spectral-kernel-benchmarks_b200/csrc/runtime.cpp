@@ -12,6 +12,9 @@
 namespace skb {
 
 void throw_cuda(cudaError_t err, const char* what) {
+    // The failure is reported by this exception: the code that the runtime keeps for
+    // the thread would fail the next plain launch's cudaGetLastError() as well.
+    cudaGetLastError();
     const int code = err == cudaErrorMemoryAllocation ? -4 : -2;
     throw Error(code, std::string(what) + ": " + cudaGetErrorName(err) + " (" + cudaGetErrorString(err) + ")");
 }
