@@ -286,9 +286,18 @@ SKB_API int skb_vertical_forward_device(skb_vertical_provider* p, const void* in
 SKB_API int skb_vertical_inverse_device(skb_vertical_provider* p, const void* in_real, const void* in_imag, void* out_real,
                                 void* out_imag, void* stream);
 
+/* A tensor-core provider runs its GEMMs on the tcgen05 pipeline, or, split TF32x3
+ * with many small groups, in a form of its own (no counterpart in the reference).
+ * The query reports 1 for each direction on the pipeline; the test switch puts both
+ * directions there for the rest of the handle's life, so that the pipeline can be
+ * checked at sizes that the other form serves. */
+SKB_API int skb_vertical_uses_pipeline(const skb_vertical_provider* p, int* forward, int* inverse);
+SKB_API int skb_vertical_use_pipeline_for_test(skb_vertical_provider* p);
+
 /* Test of the failure path (no counterpart in the reference; the reference's
  * CPU GEMMs cannot wait on a device).  With enable != 0, every later launch of
- * this tensor-core (SKB_GEMM_TF32X3) provider makes its MMA lane wait first on
+ * this tensor-core (SKB_GEMM_TF32X3, SKB_GEMM_BF16X3) provider runs the tcgen05
+ * pipeline, the form with device waits, and makes its MMA lane wait first on
  * a device barrier that nothing signals.  That wait is bounded like every wait
  * of the kernel, so it runs out: the kernel records the expiry, every role of
  * every CTA stops, outstanding copies are drained and TMEM is freed, and the

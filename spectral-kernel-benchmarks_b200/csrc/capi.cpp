@@ -1432,6 +1432,22 @@ int skb_vertical_load_modal_input_split(skb_vertical_provider* p, const double* 
     });
 }
 
+int skb_vertical_uses_pipeline(const skb_vertical_provider* p, int* forward, int* inverse) {
+    return guard([&] {
+        require(p && forward && inverse, "handle and outputs must be non-null");
+        *forward = p->forward && p->forward->uses_pipeline() ? 1 : 0;
+        *inverse = p->inverse && p->inverse->uses_pipeline() ? 1 : 0;
+    });
+}
+
+int skb_vertical_use_pipeline_for_test(skb_vertical_provider* p) {
+    return guard([&] {
+        require(p != nullptr, "handle must be non-null");
+        for (auto* plan : {p->forward.get(), p->inverse.get()})
+            if (plan) plan->use_pipeline_for_test();
+    });
+}
+
 int skb_vertical_expire_wait_for_test(skb_vertical_provider* p, int enable) {
     return guard([&] {
         require(p != nullptr, "handle must be non-null");

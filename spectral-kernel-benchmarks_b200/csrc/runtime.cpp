@@ -346,42 +346,23 @@ VerticalPlan::VerticalPlan(GemmPrecision p, int rowsOut, int inner, const std::v
             throw Error(-2, "unsupported: tensor-core GEMM needs the padded group matrix and two data stages in "
                             "227 KB of shared memory (R=" + std::to_string(rowsOut) + ", S=" + std::to_string(inner) +
                             ")");
-        error_.allocate(sizeof(int));
-        check_cuda(cudaMemset(error_.get(), 0, sizeof(int)), "cudaMemset");
         smallGroups_ = p == GemmPrecision::tf32x3 && tf32_small_groups(rowsOut, inner, groups, fields, batch);
     }
-    if (tensor_core() && !smallGroups_) {
-        // FP32 matrices (one, if common to all groups) -> the kernel's
-        // operand images, split into TF32 hi/lo or BF16 h/m/l and swizzled
-        // once here.
-        std::vector<float> f(natural.begin(), natural.end());
-        const DeviceBuffer staged = upload_vector(f);
-        const int images = static_cast<int>(groupsCount);
-        imageStride_ = common ? 0 : static_cast<long long>(tc_gemm_image_bytes(rowsOut, inner));
-        matrices_.allocate(static_cast<size_t>(images) * tc_gemm_image_bytes(rowsOut, inner));
-        check_cuda(tc_gemm_build_images(staged.get<float>(), images, rowsOut, inner,
-                                        p == GemmPrecision::bf16x3 ? 1 : 0, matrices_.get(), nullptr),
-                   "tensor-core GEMM operand images");
-        check_cuda(cudaStreamSynchronize(nullptr), "tensor-core GEMM operand images");
-        std::vector<int> gc(groups.size()), gf(groups.size());
-        for (std::uint64_t gi = 0; gi < groups.size(); ++gi) {
-            gc[gi] = static_cast<int>(groups[gi].count * fields);
-            gf[gi] = static_cast<int>(groups[gi].first * fields);
-        }
-        groupColumnsHost_ = gc;
-        build_units(tc_gemm_unit_tiles());
-        groupColumns_ = upload_vector(gc);
-        groupFirst_ = upload_vector(gf);
-        return;
-    }
-
-    const int width = gemm_tile_columns(p);
     std::vector<int> gc(groups.size()), gf(groups.size());
     for (std::uint64_t gi = 0; gi < groups.size(); ++gi) {
         gc[gi] = static_cast<int>(groups[gi].count * fields);
         gf[gi] = static_cast<int>(groups[gi].first * fields);
     }
     groupColumnsHost_ = gc;
+    groupColumns_ = upload_vector(gc);
+    groupFirst_ = upload_vector(gf);
+    if (tensor_core() && !smallGroups_) {
+        unitTiles_ = tc_gemm_unit_tiles();
+        build_pipeline(std::vector<float>(natural.begin(), natural.end()));
+        return;
+    }
+
+    const int width = gemm_tile_columns(p);
     // Member tiles unless they would run under 90 % full in a plan of several
     // members; then virtual tiles over each group's member-concatenated columns
     // (measured at 512², Nz 129, 8 members, FP64: forward 6.1 -> 4.5 ms with 4
@@ -441,8 +422,49 @@ VerticalPlan::VerticalPlan(GemmPrecision p, int rowsOut, int inner, const std::v
         matrices_ = upload_vector(At);
         matrixStride_ = common ? 0 : static_cast<long long>(matrixElems);
     }
-    groupColumns_ = upload_vector(gc);
-    groupFirst_ = upload_vector(gf);
+}
+
+// The tcgen05 form's part of a plan: FP32 matrices (one, if common to all
+// groups) -> the kernel's operand images, split into TF32 hi/lo or BF16 h/m/l and
+// swizzled once here; the work units; the word that an expired wait sets.
+void VerticalPlan::build_pipeline(const std::vector<float>& natural) {
+    const auto matrixElems = static_cast<size_t>(R_) * S_;
+    const int images = static_cast<int>(natural.size() / matrixElems);
+    const DeviceBuffer staged = upload_vector(natural);
+    imageStride_ = images == 1 && groups() > 1 ? 0 : static_cast<long long>(tc_gemm_image_bytes(R_, S_));
+    matrices_.allocate(static_cast<size_t>(images) * tc_gemm_image_bytes(R_, S_));
+    check_cuda(tc_gemm_build_images(staged.get<float>(), images, R_, S_, p_ == GemmPrecision::bf16x3 ? 1 : 0,
+                                    matrices_.get(), nullptr),
+               "tensor-core GEMM operand images");
+    check_cuda(cudaStreamSynchronize(nullptr), "tensor-core GEMM operand images");
+    build_units(unitTiles_);
+    error_.allocate(sizeof(int));
+    check_cuda(cudaMemset(error_.get(), 0, sizeof(int)), "cudaMemset");
+}
+
+void VerticalPlan::use_pipeline_for_test() {
+    if (!tensor_core()) throw Error(-1, "the tcgen05 pipeline serves the tensor-core GEMM forms");
+    if (!smallGroups_) return;
+    // The matrices back from their chunks [chunk][r][s of the chunk].
+    const size_t imageElems = static_cast<size_t>(R_) * gemm_tf32_row(S_), count = matrices_.bytes() / sizeof(float);
+    std::vector<float> stored(count), natural;
+    check_cuda(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
+    check_cuda(cudaMemcpy(stored.data(), matrices_.get(), matrices_.bytes(), cudaMemcpyDeviceToHost), "cudaMemcpy D2H");
+    for (size_t image = 0; image < count; image += imageElems)
+        for (int r = 0; r < R_; ++r)
+            for (int s = 0; s < S_; ++s) {
+                const int chunk = s / kGemmTf32Chunk, left = S_ - chunk * kGemmTf32Chunk;
+                natural.push_back(stored[image + static_cast<size_t>(chunk) * gemm_tf32_chunk_row(kGemmTf32Chunk) * R_ +
+                                         static_cast<size_t>(r) * gemm_tf32_chunk_row(left) + s % kGemmTf32Chunk]);
+            }
+    build_pipeline(natural);
+    tileTables_.clear();
+    smallGroups_ = false;
+}
+
+void VerticalPlan::set_expire_wait_for_test(bool on) {
+    if (on) use_pipeline_for_test();
+    expireWaitForTest_ = on;
 }
 
 // Units: runs of up to tiles * 64 virtual (member, column) pairs of one
@@ -607,8 +629,7 @@ void VerticalPlan::execute(ComplexOperand in, ComplexOperand out, cudaStream_t s
     }
     if (smallGroups_) {
         check_cuda(launch_grouped_gemm_tf32(R_, S_, matrices_.get<float>(), t, static_cast<const float2*>(in.re),
-                                            static_cast<float2*>(out.re), ib, ob, error_.get<int>(),
-                                            expireWaitForTest_, s),
+                                            static_cast<float2*>(out.re), ib, ob, s),
                    "split-TF32x3 grouped vertical GEMM kernel");
         return;
     }

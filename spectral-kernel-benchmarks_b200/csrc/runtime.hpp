@@ -192,11 +192,16 @@ public:
     // dense bin array instead of compact [column][len] arrays.
     void execute(ComplexOperand in, ComplexOperand out, cudaStream_t s, std::uint64_t members = 0,
                  const BinBoundary* inBins = nullptr, const BinBoundary* outBins = nullptr) const;
-    // Raises if a bounded device wait of the tensor-core form expired.
+    // Raises if a bounded device wait of the tcgen05 pipeline expired.
     void check_device_error() const;
-    // Tensor-core form: the next launches wait on a device barrier that
-    // nothing signals, so their bounded wait expires (tests the error path).
-    void set_expire_wait_for_test(bool on) { expireWaitForTest_ = on; }
+    // Whether the plan runs the tcgen05 pipeline (tc_gemm.cu), which alone has waits.
+    bool uses_pipeline() const { return tensor_core() && !smallGroups_; }
+    // Tests of that kernel at sizes that the small-group form serves: the plan runs
+    // it from now on (device work must not be in flight on the plan).
+    void use_pipeline_for_test();
+    // Tensor-core form: the next launches, of the pipeline, wait on a device barrier
+    // that nothing signals, so their bounded wait expires (tests the error path).
+    void set_expire_wait_for_test(bool on);
     GemmPrecision precision() const { return p_; }
     // The split TF32x3 and BF16x3 forms run on the tcgen05 tensor cores.
     bool tensor_core() const { return p_ == GemmPrecision::tf32x3 || p_ == GemmPrecision::bf16x3; }
@@ -213,6 +218,7 @@ public:
     std::uint64_t groups() const { return groupColumnsHost_.size(); }
 
 private:
+    void build_pipeline(const std::vector<float>& natural);
     void build_units(int tiles);
     GemmPrecision p_;
     int R_, S_;

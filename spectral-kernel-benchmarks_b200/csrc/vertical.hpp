@@ -144,8 +144,8 @@ constexpr int gemm_tf32_row(int S) {
 cudaError_t gemm_tf32_build_images(const float* natural, long long groups, int R, int S, float* images,
                                    cudaStream_t stream);
 cudaError_t launch_grouped_gemm_tf32(int R, int S, const float* images, const GroupTiles& tiles, const float2* in,
-                                     float2* out, const BinBoundary& inBins, const BinBoundary& outBins, int* error,
-                                     bool expireWaitForTest, cudaStream_t stream);
+                                     float2* out, const BinBoundary& inBins, const BinBoundary& outBins,
+                                     cudaStream_t stream);
 
 // inBins / outBins (optional): cell-addressed operands (BinBoundary) instead of
 // the compact [column][len] arrays.

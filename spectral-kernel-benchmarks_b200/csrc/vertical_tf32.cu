@@ -124,33 +124,13 @@ template <int MH>
 __global__ void __launch_bounds__(kThreads, resident<MH>())
     grouped_gemm_tf32_kernel(int R, int S, const float* __restrict__ images, GroupTiles tiles,
                              const float2* __restrict__ in, float2* __restrict__ out, BinBoundary inBins,
-                             BinBoundary outBins, int* error, int expireWaitForTest) {
+                             BinBoundary outBins) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     // Element offsets of each tile column's input and output (and the output
     // partner, or -1), and whether the output is conjugated.
     __shared__ long long colIn[kTileCols], colOut[kTileCols], colPartner[kTileCols];
     __shared__ bool colConj[kTileCols];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (expireWaitForTest != 0) {
-        // Failure-path test of the provider: a bounded wait on a barrier that
-        // nothing arrives on runs out and is reported; nothing is computed.
-        __shared__ __align__(8) unsigned long long never;
-        if (tid == 0) {
-            const unsigned bar = static_cast<unsigned>(__cvta_generic_to_shared(&never));
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
-            unsigned done = 0;
-            for (int i = 0; i < (1 << 14) && done == 0; ++i)
-                asm volatile(
-                    "{\n\t.reg .pred p;\n\t"
-                    "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\t"
-                    "selp.u32 %0, 1, 0, p;\n\t}"
-                    : "=r"(done)
-                    : "r"(bar)
-                    : "memory");
-            if (done == 0) atomicExch(error, 1);
-        }
-        return;
-    }
     const int tile = blockIdx.x;
     const int g = __ldg(tiles.tileGroup + tile);
     const int c0 = __ldg(tiles.tileColumn + tile);
@@ -263,7 +243,7 @@ __global__ void __launch_bounds__(kThreads, resident<MH>())
 
 template <int MH>
 cudaError_t launch_mh(int R, int S, const float* images, const GroupTiles& tiles, const float2* in, float2* out,
-                      const BinBoundary& ib, const BinBoundary& ob, int* error, int expire, cudaStream_t stream) {
+                      const BinBoundary& ib, const BinBoundary& ob, cudaStream_t stream) {
     auto kernel = grouped_gemm_tf32_kernel<MH>;
     const size_t bytes = 2 * stage_bytes<MH>();
     if (bytes > 48 * 1024) {
@@ -271,7 +251,7 @@ cudaError_t launch_mh(int R, int S, const float* images, const GroupTiles& tiles
         if (err != cudaSuccess) return err;
     }
     return launch_chained(kernel, dim3(unsigned(tiles.tiles)), kThreads, bytes, stream, R, S, images, tiles, in, out, ib,
-                          ob, error, expire);
+                          ob);
 }
 
 // natural [groups][R][S] -> images, one thread per (group, row, s of the padded row).
@@ -304,16 +284,15 @@ cudaError_t gemm_tf32_build_images(const float* natural, long long groups, int R
 }
 
 cudaError_t launch_grouped_gemm_tf32(int R, int S, const float* images, const GroupTiles& tiles, const float2* in,
-                                     float2* out, const BinBoundary& ib, const BinBoundary& ob, int* error,
-                                     bool expireWaitForTest, cudaStream_t stream) {
+                                     float2* out, const BinBoundary& ib, const BinBoundary& ob,
+                                     cudaStream_t stream) {
     if (tiles.tiles <= 0) return cudaSuccess;
-    const int expire = expireWaitForTest ? 1 : 0;
     switch (((R + 15) / 16 + 1) / 2) {
-        case 1: return launch_mh<1>(R, S, images, tiles, in, out, ib, ob, error, expire, stream);
-        case 2: return launch_mh<2>(R, S, images, tiles, in, out, ib, ob, error, expire, stream);
-        case 3: return launch_mh<3>(R, S, images, tiles, in, out, ib, ob, error, expire, stream);
-        case 4: return launch_mh<4>(R, S, images, tiles, in, out, ib, ob, error, expire, stream);
-        case 5: return launch_mh<5>(R, S, images, tiles, in, out, ib, ob, error, expire, stream);
+        case 1: return launch_mh<1>(R, S, images, tiles, in, out, ib, ob, stream);
+        case 2: return launch_mh<2>(R, S, images, tiles, in, out, ib, ob, stream);
+        case 3: return launch_mh<3>(R, S, images, tiles, in, out, ib, ob, stream);
+        case 4: return launch_mh<4>(R, S, images, tiles, in, out, ib, ob, stream);
+        case 5: return launch_mh<5>(R, S, images, tiles, in, out, ib, ob, stream);
         default: return cudaErrorInvalidValue;
     }
 }
