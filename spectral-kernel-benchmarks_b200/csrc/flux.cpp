@@ -156,7 +156,7 @@ FluxPipeline::FluxPipeline(const FluxConfig& cfg) : cfg_(cfg) {
         }
     } else {
         shared_.allocate(es * 3 * cfg.members * volume_);
-        target_.allocate(horizontal_->blocked_bytes(cfg.members * cfg.nz));
+        target_.allocate(horizontal_->bin_bytes(cfg.members * cfg.nz));
     }
     allocationSeconds = seconds_since(allocStart) + horizontal_->allocationSeconds;
     planningSeconds += horizontal_->planningSeconds;
@@ -503,9 +503,10 @@ void FluxPipeline::run(const void* modalIn, void* modalOut, cudaStream_t s, Reco
     horizontal_->inverse_rows(shared_.get(), 3 * M * nz, s);
     if (rec) rec->end("rows_inverse_c2r", 1, triplePlanes * (binsPlane + realPlane), 0.0);
     const double scale = 1.0 / (n * n * n * n);
+    const DenseBins target = horizontal_->bin_array(target_.get(), cfg_.members * nz);
     for (std::uint64_t t = 0; t < T; ++t) {
         inverseColumns(3 + 3 * t);
-        horizontal_->product_rows(shared_.get(), M, scale, target_.get(), s);
+        horizontal_->product_rows(shared_.get(), M, scale, target, s);
         if (rec)
             rec->end("rows_product", 1, triplePlanes * (binsPlane + realPlane) + double(M) * nz * binsPlane,
                      6.0 * double(volume_) * M);
@@ -513,7 +514,7 @@ void FluxPipeline::run(const void* modalIn, void* modalOut, cudaStream_t s, Reco
         out.count = static_cast<int>(M);
         for (std::uint64_t m = 0; m < M; ++m)
             out.v[m] = {physOut + ces * ((m * H * T + t) * nz), nullptr, static_cast<long long>(T * nz)};
-        horizontal_->forward_columns(target_.get(), out, 1.0, s);
+        horizontal_->forward_columns(target, out, 1.0, s);
         if (rec) rec->end("columns_forward_gather", 1, double(M) * nz * (binsPlane + compactPlane), 0.0);
     }
     gemm_forward(modalOut, s, M, false);

@@ -110,7 +110,7 @@ HorizontalPlan::HorizontalPlan(const Workload& w, Precision p, bool pruned, std:
     modeKx_ = upload_vector(tables.modeKx);
     modeKy_ = upload_vector(tables.modeKy);
     modeConj_ = upload_vector(tables.modeConj);
-    bins_.allocate(blocked_bytes(maxPlanes));
+    bins_.allocate(bin_bytes(maxPlanes));
     {
         // Per-column band of the retained cells, and whether it is exact.
         std::vector<int> band(static_cast<size_t>(keep_), -1);
@@ -144,7 +144,7 @@ ModeTables HorizontalPlan::tables() const {
 void HorizontalPlan::forward_rows(const void* real, std::uint64_t planes, cudaStream_t s) const {
     if (planes > maxPlanes_) throw Error(-1, "plane count exceeds the plan's scratch");
     check_cuda(launch_rows_forward(p_, static_cast<int>(w_.nx), static_cast<int>(w_.ny),
-                                   static_cast<long long>(planes), keep_, real, scratch(planes), rowForward_.get(),
+                                   static_cast<long long>(planes), keep_, real, scratch(), rowForward_.get(),
                                    twFull_.get(), s),
                "row r2c kernel");
 }
@@ -152,21 +152,21 @@ void HorizontalPlan::forward_rows(const void* real, std::uint64_t planes, cudaSt
 void HorizontalPlan::forward_columns(const ViewSet& views, double scale, cudaStream_t s) const {
     if (static_cast<std::uint64_t>(views.count) * w_.nz > maxPlanes_)
         throw Error(-1, "plane count exceeds the plan's scratch");
-    forward_columns(bins_.get(), views, scale, s);
+    forward_columns(scratch(), views, scale, s);
 }
 
-void HorizontalPlan::forward_columns(const void* target, const ViewSet& views, double scale, cudaStream_t s) const {
-    check_cuda(launch_columns_gather(p_, static_cast<int>(w_.ny), static_cast<int>(w_.nz), keep_,
-                                     blocked(const_cast<void*>(target)), views, tables(), scale, colTable_.get(), s),
+void HorizontalPlan::forward_columns(DenseBins in, const ViewSet& views, double scale, cudaStream_t s) const {
+    check_cuda(launch_columns_gather(p_, static_cast<int>(w_.ny), static_cast<int>(w_.nz), keep_, in, views, tables(),
+                                     scale, colTable_.get(), s),
                "column c2c + retention kernel");
 }
 
-void HorizontalPlan::product_rows(const void* velocity, std::uint64_t members, double scale, void* target,
+void HorizontalPlan::product_rows(const void* velocity, std::uint64_t members, double scale, DenseBins target,
                                   cudaStream_t s) const {
     if (3 * members * w_.nz > maxPlanes_) throw Error(-1, "plane count exceeds the plan's scratch");
     check_cuda(launch_rows_product(p_, static_cast<int>(w_.nx), static_cast<int>(w_.ny), static_cast<int>(w_.nz),
-                                   static_cast<int>(members), keep_, scale, velocity, blocked(bins_.get()),
-                                   blocked(target), rowInverse_.get(), rowForward_.get(), twFull_.get(), s),
+                                   static_cast<int>(members), keep_, scale, velocity, scratch(), target,
+                                   rowInverse_.get(), rowForward_.get(), twFull_.get(), s),
                "row product kernel");
 }
 
@@ -174,7 +174,7 @@ void HorizontalPlan::inverse_columns(const ViewSet& views, cudaStream_t s) const
     const auto planes = static_cast<std::uint64_t>(views.count) * w_.nz;
     if (planes > maxPlanes_) throw Error(-1, "plane count exceeds the plan's scratch");
     check_cuda(launch_columns_embed(p_, static_cast<int>(w_.ny), static_cast<int>(w_.nz), keep_, views, tables(),
-                                    scratch(planes), colTable_.get(), s),
+                                    scratch(), colTable_.get(), s),
                "embedding + column c2c kernel");
 }
 
@@ -231,7 +231,7 @@ void HorizontalPlan::forward_columns_band(DenseBins bins, int slots, double scal
 void HorizontalPlan::inverse_rows(void* real, std::uint64_t planes, cudaStream_t s) const {
     if (planes > maxPlanes_) throw Error(-1, "plane count exceeds the plan's scratch");
     check_cuda(launch_rows_inverse(p_, static_cast<int>(w_.nx), static_cast<int>(w_.ny),
-                                   static_cast<long long>(planes), keep_, scratch(planes), real, rowInverse_.get(),
+                                   static_cast<long long>(planes), keep_, scratch(), real, rowInverse_.get(),
                                    twFull_.get(), s),
                "row c2r kernel");
 }
@@ -265,10 +265,10 @@ void HorizontalPlan::inverse_dense(const void* wvm, void* real, std::uint64_t pl
     if (planes > maxPlanes_) throw Error(-1, "plane count exceeds the plan's scratch");
     const DenseBins in{const_cast<void*>(wvm), static_cast<long long>(planes), static_cast<long long>(w_.nxHalf())};
     check_cuda(launch_columns_dense(p_, +1, static_cast<int>(w_.ny), keep_, static_cast<long long>(planes), in,
-                                    scratch(planes), colTable_.get(), s),
+                                    scratch(), colTable_.get(), s),
                "column c2c kernel");
     check_cuda(launch_rows_inverse(p_, static_cast<int>(w_.nx), static_cast<int>(w_.ny),
-                                   static_cast<long long>(planes), keep_, scratch(planes), real, rowInverse_.get(),
+                                   static_cast<long long>(planes), keep_, scratch(), real, rowInverse_.get(),
                                    twFull_.get(), s),
                "row c2r kernel");
 }

@@ -12,6 +12,7 @@
 
 #include <cuda_runtime.h>
 
+#include "bin_layout.hpp"
 #include "horizontal.hpp"
 #include "model.hpp"
 #include "vertical.hpp"
@@ -101,20 +102,17 @@ public:
     int keep() const { return keep_; }
     std::uint64_t modes() const { return modeCount_; }
     ModeTables tables() const;
-    // The scratch is plane-blocked.
-    std::uint64_t scratch_blocks(std::uint64_t planes) const {
-        return (planes + (std::uint64_t(1) << kScratchShift) - 1) >> kScratchShift;
+    // Bin arrays of a plan (bin_layout.hpp): its scratch, and others of the same rows.
+    std::uint64_t bin_bytes(std::uint64_t planes) const {
+        return bin_array_bytes(w_.ny, static_cast<std::uint64_t>(keep_), planes, element_bytes(p_));
     }
-    DenseBins scratch(std::uint64_t) const { return blocked(bins_.get()); }
-    std::uint64_t blocked_bytes(std::uint64_t planes) const {
-        return w_.ny * static_cast<std::uint64_t>(keep_) * (scratch_blocks(planes) << kScratchShift) * 2 *
-               element_bytes(p_);
-    }
-    DenseBins blocked(void* data) const {
-        const long long block = 1LL << kScratchShift;
-        return {data, block, static_cast<long long>(keep_), kScratchShift,
+    DenseBins bin_array(void* data, std::uint64_t planes) const {
+        if (planes < kBinBlock) return {data, static_cast<long long>(planes), static_cast<long long>(keep_)};
+        const long long block = static_cast<long long>(kBinBlock);
+        return {data, block, static_cast<long long>(keep_), kBinBlockShift,
                 block * static_cast<long long>(keep_) * static_cast<long long>(w_.ny)};
     }
+    DenseBins scratch() const { return bin_array(bins_.get(), maxPlanes_); }
 
     // x then y (forward) into views; y then x (inverse) from views.
     void forward(const void* real, std::uint64_t planes, const ViewSet& views, double scale, cudaStream_t s) const;
@@ -124,9 +122,9 @@ public:
     void inverse_columns(const ViewSet& views, cudaStream_t s) const;
     void inverse_rows(void* real, std::uint64_t planes, cudaStream_t s) const;
     // Flux target of the derivative slots in the scratch (launch_rows_product), and
-    // its column stage; `target` holds blocked_bytes(members * Nz) bytes.
-    void product_rows(const void* velocity, std::uint64_t members, double scale, void* target, cudaStream_t s) const;
-    void forward_columns(const void* target, const ViewSet& views, double scale, cudaStream_t s) const;
+    // its column stage; `target` is a bin array of members * Nz planes.
+    void product_rows(const void* velocity, std::uint64_t members, double scale, DenseBins target, cudaStream_t s) const;
+    void forward_columns(DenseBins in, const ViewSet& views, double scale, cudaStream_t s) const;
     // Full-grid dense forms (keep = Nx/2+1): WVM spectrum with `planes` planes.
     void forward_dense(const void* real, void* wvm, std::uint64_t planes, cudaStream_t s) const;
     void inverse_dense(const void* wvm, void* real, std::uint64_t planes, cudaStream_t s) const;
@@ -169,7 +167,6 @@ private:
     DeviceBuffer cellMap_, gatherMap_, colStart_, colKy_, colMode_, modeKx_, modeKy_, modeConj_;
     DeviceBuffer bins_;
     DeviceBuffer band_;
-    static constexpr int kScratchShift = 4;
     bool bandExact_ = false;
     int bandFormInverse_ = 0, bandFormForward_ = 0;
 };
