@@ -66,19 +66,34 @@ FluxPipeline::FluxPipeline(const FluxConfig& cfg) : cfg_(cfg) {
                                                                   : GemmPrecision::f32;
     const size_t es = element_bytes(hp);
     fused_ = split && rows_flux_supported(static_cast<long long>(cfg.n));
-    // Admission by device memory: refuse before allocating what cannot fit.
-    const std::uint64_t maxPlanes = fused_ ? 1 : 3 * cfg.members * cfg.nz;
-    const std::uint64_t binPlanes = fused_ ? cfg.members * cfg.nz * (fieldsIn_ + cfg.targets) : maxPlanes;
-    std::uint64_t need = 2 * es * cfg.members * modes_ * cfg.nz * (fieldsIn_ + cfg.targets)  // physIn, physOut
-                         + (fused_ ? 0 : es * volume_ * cfg.members * 7)                   // bound of U, V, W and target bins
-                         + 2 * es * cfg.n * (cfg.n / 2 + 1) * binPlanes * 9 / 8;           // bin scratch bound
+    // The fused path's plan is small (one plane) and tells whether the dense boundary serves.
+    auto makeHorizontal = [&](std::uint64_t planes) {
+        horizontal_ = std::make_unique<HorizontalPlan>(Workload{cfg.n, cfg.n, cfg.nz, 3, 1.0, 1.0, true}, hp, true,
+                                                       planes);
+    };
+    if (fused_) makeHorizontal(1);
+    dense_ = fused_ && horizontal_->band_exact();
+    // Bin planes per slot of the fused path, padded to a multiple of 8 (64 bytes of
+    // FP32 complex), so every 8-plane run a column or row CTA moves starts on a
+    // 64-byte boundary.
+    zStride_ = (cfg.nz + 7) / 8 * 8;
+    // Admission by device memory: refuse before allocating what cannot fit.  Counted
+    // are the scratch arrays below and the matrices, unpadded, of both directions.
+    const std::uint64_t slots = fieldsIn_ + cfg.targets, keep = active_columns(modes);
+    std::uint64_t need = 2 * es * groups.size() * nj_ * cfg.nz;
+    if (!dense_) need += 2 * es * cfg.members * modes_ * cfg.nz * slots;  // physIn_, physOut_
+    if (fused_)
+        need += 2 * es * cfg.n * keep * cfg.members * slots * zStride_;  // binsIn_, binsOut_
+    else
+        need += es * 3 * cfg.members * volume_ +  // U, V, W, the scratch and the target's bins
+                bin_array_bytes(cfg.n, keep, 3 * cfg.members * cfg.nz, es) +
+                bin_array_bytes(cfg.n, keep, cfg.members * cfg.nz, es);
     size_t freeBytes = 0, totalBytes = 0;
     check_cuda(cudaMemGetInfo(&freeBytes, &totalBytes), "cudaMemGetInfo");
     if (need > freeBytes)
         throw Error(-4, "flux workload needs " + std::to_string(need) + " device bytes; " +
                             std::to_string(freeBytes) + " are free");
-    horizontal_ = std::make_unique<HorizontalPlan>(Workload{cfg.n, cfg.n, cfg.nz, 3, 1.0, 1.0, true}, hp, true,
-                                                   maxPlanes);
+    if (!fused_) makeHorizontal(3 * cfg.members * cfg.nz);
     if (!families_) {
         inverseGemm_ = std::make_unique<VerticalPlan>(gp, static_cast<int>(cfg.nz), static_cast<int>(nj_), groups,
                                                       fieldsIn_, cfg.members, fam.inverse, kGemmBatch);
@@ -119,17 +134,11 @@ FluxPipeline::FluxPipeline(const FluxConfig& cfg) : cfg_(cfg) {
         cellPhysIn_ = upload_vector(pi);
         cellPhysOut_ = upload_vector(po);
     }
-    dense_ = fused_ && horizontal_->band_exact();
     if (!dense_) {
         physIn_.allocate(2 * es * cfg.members * modes_ * fieldsIn_ * cfg.nz);
         physOut_.allocate(2 * es * cfg.members * modes_ * cfg.targets * cfg.nz);
     }
     if (fused_) {
-        // Bin planes per slot padded to a multiple of 8 (64 bytes of FP32
-        // complex), so every 8-plane run a column or row CTA moves starts on a
-        // 64-byte boundary.
-        zStride_ = (cfg.nz + 7) / 8 * 8;
-        const std::uint64_t keep = static_cast<std::uint64_t>(horizontal_->keep());
         binsIn_.allocate(2 * es * cfg.n * keep * cfg.members * fieldsIn_ * zStride_);
         binsOut_.allocate(2 * es * cfg.n * keep * cfg.members * cfg.targets * zStride_);
         rowsError_.allocate(sizeof(int));

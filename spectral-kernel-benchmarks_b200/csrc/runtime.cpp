@@ -67,13 +67,11 @@ DeviceBuffer upload_real_table(const std::vector<double>& values, Precision p) {
     return upload_vector(f);
 }
 
-namespace {
 std::uint64_t active_columns(const std::vector<RetainedMode>& modes) {
     std::uint64_t active = 0;
     for (const auto& m : modes) active = std::max<std::uint64_t>(active, m.kx + 1);
     return active;
 }
-}  // namespace
 
 HorizontalPlan::HorizontalPlan(const Workload& w, Precision p, bool pruned, std::uint64_t maxPlanes)
     : w_(w), p_(p), maxPlanes_(maxPlanes) {

@@ -91,6 +91,9 @@ std::vector<double> regs_table(const std::vector<double>& natural, int perThread
 // Upload a double table in the plan's precision.
 DeviceBuffer upload_real_table(const std::vector<double>& values, Precision p);
 
+// kx columns that hold retained modes: a pruned plan keeps kx below this.
+std::uint64_t active_columns(const std::vector<RetainedMode>& modes);
+
 // Horizontal plan: twiddles, column tables and the dense bin scratch for a
 // grid, a kept kx band and a maximum plane count.
 class HorizontalPlan {

@@ -1,6 +1,7 @@
 """Plans of few planes: their bin arrays are blocks of 16 planes from 16 planes on and
 hold just the plan's planes below.  Sizes of the scratch, and results on both sides of
-that line (a flux's target array may lie below it and its scratch above).
+that line (a flux's target array may lie below it and its scratch above).  A flux is
+refused, before anything large is allocated, by the same sizes.
 
 Tolerances as in test_gpu_horizontal.py and the flux tests: FP64 1e-12, FP32 1e-5."""
 
@@ -49,15 +50,18 @@ def test_pruned_results(nz, fields, precision, tol):
     assert orc.rel_l2_error(pruned.forward(real), orc.gather_retained(o, modes, orc.fft_r2c(o, real))) <= tol
 
 
+def _staged_bytes(n, nz, targets, members):
+    modes, keep = len(orc.retained_modes(n, n)), _keep(n)
+    planes = 3 * members * nz
+    return (16 * members * modes * nz * (3 + 4 * targets)  # physical values of every slot and target
+            + 8 * n * n * planes  # U, V and W
+            + 16 * n * keep * (_stored(planes) + _stored(members * nz)))
+
+
 @pytest.mark.parametrize("n,nz,targets,members", [(8, 3, 3, 1), (16, 3, 4, 2), (32, 5, 3, 3), (16, 15, 3, 2)])
 def test_staged_flux(n, nz, targets, members):
     flux = skb_cuda.Flux(n, nz, targets=targets, members=members)
-    modes, keep = len(orc.retained_modes(n, n)), _keep(n)
-    planes = 3 * members * nz
-    assert _info(flux)["scratch_bytes"] == (
-        16 * members * modes * nz * (3 + 4 * targets)  # physical values of every slot and target
-        + 8 * n * n * planes  # U, V and W
-        + 16 * n * keep * (_stored(planes) + _stored(members * nz)))
+    assert _info(flux)["scratch_bytes"] == _staged_bytes(n, nz, targets, members)
     rng = np.random.default_rng(n)
     x = rng.uniform(-0.125, 0.125, flux.input_elements) + 1j * rng.uniform(-0.125, 0.125, flux.input_elements)
     d_in = skb_cuda.DeviceArray.from_numpy(x)
@@ -70,3 +74,19 @@ def test_staged_flux(n, nz, targets, members):
         for m in range(active):
             ref = orc.flux(n, nz, x[m * per_in:(m + 1) * per_in], targets=targets)
             assert orc.rel_l2_error(out[m * per_out:(m + 1) * per_out], ref) <= 1e-12
+
+
+@pytest.mark.parametrize("n,nz,targets", [(64, 3, 3), (128, 9, 4), (512, 5, 3)])
+def test_fused_scratch(n, nz, targets):
+    flux = skb_cuda.Flux(n, nz, targets=targets, members=2, mode=skb_cuda.FLUX_SPLIT_TF32X3)
+    bins = 8 * n * _keep(n) * 2 * (3 + 4 * targets) * ((nz + 7) // 8 * 8)
+    assert _info(flux)["scratch_bytes"] == bins + 8 * n * _keep(n)  # and the plan's one plane
+
+
+def test_refusal_names_what_the_handle_would_hold():
+    n, nz, targets, members = 1024, 48, 4, 42  # more than any device holds
+    w = skb_cuda.Workload(n, n, nz, targets)
+    matrices = 16 * len(skb_cuda.squared_wavenumber_groups(w)) * w.nj * nz
+    with pytest.raises(MemoryError, match="flux workload needs %d device bytes" %
+                       (_staged_bytes(n, nz, targets, members) + matrices)):
+        skb_cuda.Flux(n, nz, targets=targets, members=members)
