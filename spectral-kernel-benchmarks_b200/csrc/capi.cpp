@@ -260,8 +260,7 @@ struct skb_cs_vertical {
     uint64_t rows = 0, nz = 0;
     Precision p = Precision::f64;
     cudaStream_t stream = nullptr;
-    DeviceBuffer tw;        // 2(nz-1) twiddles exp(-2 pi i m / (2(nz-1)))
-    DeviceBuffer table;     // the same in the order of the register-ended transform
+    DeviceBuffer tw;        // 2(nz-1) twiddles exp(-2 pi i m / (2(nz-1))), see launch_type1
     DeviceBuffer arena, arena1;  // device staging of host arrays
     HostAdapter host{Precision::f64, {}};
     double allocation = 0.0, planning = 0.0;
@@ -1209,7 +1208,7 @@ void type1_run(skb_cs_vertical* p, unsigned mask, uint64_t storage, uint64_t fir
                bool normalize, void* data, cudaStream_t s) {
     check_cuda(launch_type1(p->p == Precision::f64, data, static_cast<long long>(p->rows), static_cast<int>(p->nz),
                             static_cast<int>(storage), static_cast<int>(first), static_cast<int>(channels), mask,
-                            normalize, p->tw.get(), p->table.get(), s),
+                            normalize, p->tw.get(), s),
                "type-I vertical transform kernel");
 }
 
@@ -1229,9 +1228,8 @@ int skb_cs_vertical_create(uint64_t rows, uint64_t nz, int precision, skb_cs_ver
         p->stream = make_stream();
         const auto t0 = std::chrono::steady_clock::now();
         const auto tw = twiddle_table(2 * (nz - 1));
-        p->tw = upload_real_table(tw, p->p);
-        if (type1_uses_fft(static_cast<int>(nz)))
-            p->table = upload_real_table(regs_table(tw, regs_per_thread(static_cast<int>(2 * (nz - 1)))), p->p);
+        p->tw = upload_real_table(
+            type1_uses_regs(nz) ? regs_table(tw, regs_per_thread(static_cast<int>(2 * (nz - 1)))) : tw, p->p);
         p->planning = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
         *out = p.release();
     });
@@ -1249,7 +1247,7 @@ int skb_cs_vertical_info(const skb_cs_vertical* p, skb_provider_info* info) {
         std::memset(info, 0, sizeof(*info));
         info->planning_seconds = p->planning;
         info->allocation_seconds = p->allocation;
-        info->persistent_bytes = p->tw.bytes() + p->table.bytes();
+        info->persistent_bytes = p->tw.bytes();
         info->scratch_bytes = p->arena.bytes() + p->arena1.bytes();
         info->launches_per_execution = 1;
         info->precision = p->p == Precision::f64 ? SKB_PRECISION_FP64 : SKB_PRECISION_FP32;

@@ -69,7 +69,7 @@ FluxPipeline::FluxPipeline(const FluxConfig& cfg) : cfg_(cfg) {
     // The fused path's plan is small (one plane) and tells whether the dense boundary serves.
     auto makeHorizontal = [&](std::uint64_t planes) {
         horizontal_ = std::make_unique<HorizontalPlan>(Workload{cfg.n, cfg.n, cfg.nz, 3, 1.0, 1.0, true}, hp, true,
-                                                       planes);
+                                                       planes, fused_);
     };
     if (fused_) makeHorizontal(1);
     dense_ = fused_ && horizontal_->band_exact();

@@ -73,7 +73,7 @@ std::uint64_t active_columns(const std::vector<RetainedMode>& modes) {
     return active;
 }
 
-HorizontalPlan::HorizontalPlan(const Workload& w, Precision p, bool pruned, std::uint64_t maxPlanes)
+HorizontalPlan::HorizontalPlan(const Workload& w, Precision p, bool pruned, std::uint64_t maxPlanes, bool fused)
     : w_(w), p_(p), maxPlanes_(maxPlanes) {
     validate_workload(w);
     if (!supported_length(static_cast<long long>(w.nx)) || !supported_length(static_cast<long long>(w.ny)))
@@ -92,14 +92,25 @@ HorizontalPlan::HorizontalPlan(const Workload& w, Precision p, bool pruned, std:
     planningSeconds = seconds_since(planStart);
 
     const auto allocStart = Clock::now();
-    twHalf_ = upload_real_table(twHalf, p);
-    twFull_ = upload_real_table(twFull, p);
-    twCol_ = upload_real_table(twCol, p);
+    // The twiddle tables that the path reads, in one buffer and one copy.
     const int half = static_cast<int>(std::max<std::uint64_t>(1, w.nx / 2));
-    rowForward_ = upload_real_table(regs_table(twHalf, row_regs_per_thread(half)), p);
-    rowInverse_ = upload_real_table(regs_table(twHalf, row_regs_per_thread(half), row_plane_radix(half)), p);
-    colTable_ = upload_real_table(
-        regs_table(twCol, column_regs_per_thread(static_cast<int>(w.ny), p == Precision::f64)), p);
+    std::vector<double> twiddles;
+    std::vector<std::pair<const void**, size_t>> placed;
+    auto place = [&](const void** table, const std::vector<double>& values) {
+        placed.push_back({table, twiddles.size() * element_bytes(p)});
+        twiddles.insert(twiddles.end(), values.begin(), values.end());
+    };
+    place(&twFull_, twFull);
+    place(&colTable_, regs_table(twCol, column_regs_per_thread(static_cast<int>(w.ny), p == Precision::f64)));
+    if (fused) {
+        place(&twHalf_, twHalf);
+        place(&twCol_, twCol);
+    } else {
+        place(&rowForward_, regs_table(twHalf, row_regs_per_thread(half)));
+        place(&rowInverse_, regs_table(twHalf, row_regs_per_thread(half), row_plane_radix(half)));
+    }
+    twiddles_ = upload_real_table(twiddles, p);
+    for (const auto& [table, offset] : placed) *table = twiddles_.get<unsigned char>() + offset;
     cellMap_ = upload_vector(tables.cellMap);
     gatherMap_ = upload_vector(tables.gatherMap);
     colStart_ = upload_vector(tables.colStart);
@@ -129,8 +140,7 @@ HorizontalPlan::HorizontalPlan(const Workload& w, Precision p, bool pruned, std:
         band_ = upload_vector(band);
     }
     allocationSeconds = seconds_since(allocStart);
-    persistentBytes = twHalf_.bytes() + twFull_.bytes() + twCol_.bytes() + rowForward_.bytes() + rowInverse_.bytes() + colTable_.bytes() + cellMap_.bytes() + gatherMap_.bytes() +
-                      colStart_.bytes() +
+    persistentBytes = twiddles_.bytes() + cellMap_.bytes() + gatherMap_.bytes() + colStart_.bytes() +
                       colKy_.bytes() + colMode_.bytes() + modeKx_.bytes() + modeKy_.bytes() + modeConj_.bytes();
     scratchBytes = bins_.bytes();
 }
@@ -142,8 +152,8 @@ ModeTables HorizontalPlan::tables() const {
 void HorizontalPlan::forward_rows(const void* real, std::uint64_t planes, cudaStream_t s) const {
     if (planes > maxPlanes_) throw Error(-1, "plane count exceeds the plan's scratch");
     check_cuda(launch_rows_forward(p_, static_cast<int>(w_.nx), static_cast<int>(w_.ny),
-                                   static_cast<long long>(planes), keep_, real, scratch(), rowForward_.get(),
-                                   twFull_.get(), s),
+                                   static_cast<long long>(planes), keep_, real, scratch(), rowForward_,
+                                   twFull_, s),
                "row r2c kernel");
 }
 
@@ -155,7 +165,7 @@ void HorizontalPlan::forward_columns(const ViewSet& views, double scale, cudaStr
 
 void HorizontalPlan::forward_columns(DenseBins in, const ViewSet& views, double scale, cudaStream_t s) const {
     check_cuda(launch_columns_gather(p_, static_cast<int>(w_.ny), static_cast<int>(w_.nz), keep_, in, views, tables(),
-                                     scale, colTable_.get(), s),
+                                     scale, colTable_, s),
                "column c2c + retention kernel");
 }
 
@@ -164,7 +174,7 @@ void HorizontalPlan::product_rows(const void* velocity, std::uint64_t members, d
     if (3 * members * w_.nz > maxPlanes_) throw Error(-1, "plane count exceeds the plan's scratch");
     check_cuda(launch_rows_product(p_, static_cast<int>(w_.nx), static_cast<int>(w_.ny), static_cast<int>(w_.nz),
                                    static_cast<int>(members), keep_, scale, velocity, scratch(), target,
-                                   rowInverse_.get(), rowForward_.get(), twFull_.get(), s),
+                                   rowInverse_, rowForward_, twFull_, s),
                "row product kernel");
 }
 
@@ -172,7 +182,7 @@ void HorizontalPlan::inverse_columns(const ViewSet& views, cudaStream_t s) const
     const auto planes = static_cast<std::uint64_t>(views.count) * w_.nz;
     if (planes > maxPlanes_) throw Error(-1, "plane count exceeds the plan's scratch");
     check_cuda(launch_columns_embed(p_, static_cast<int>(w_.ny), static_cast<int>(w_.nz), keep_, views, tables(),
-                                    scratch(), colTable_.get(), s),
+                                    scratch(), colTable_, s),
                "embedding + column c2c kernel");
 }
 
@@ -182,13 +192,13 @@ void HorizontalPlan::inverse_columns_into(const ViewSet& views, DenseBins out, c
     if (zStride == 0) zStride = nz;
     if (p_ == Precision::f32 && columns_warp_supported(static_cast<long long>(w_.ny))) {
         check_cuda(launch_columns_embed_warp(static_cast<int>(w_.ny), nz, zStride, keep_, views, tables(), out,
-                                             twCol_.get(), s),
+                                             twCol_, s),
                    "warp embedding + column c2c kernel");
         return;
     }
     if (zStride != nz) throw Error(-3, "padded bin planes need the FP32 warp column kernels");
     check_cuda(launch_columns_embed(p_, static_cast<int>(w_.ny), static_cast<int>(w_.nz), keep_, views, tables(), out,
-                                    colTable_.get(), s),
+                                    colTable_, s),
                "embedding + column c2c kernel");
 }
 
@@ -199,13 +209,13 @@ void HorizontalPlan::forward_columns_from(DenseBins in, const ViewSet& views, do
     if (zStride == 0) zStride = nz;
     if (p_ == Precision::f32 && columns_warp_supported(static_cast<long long>(w_.ny))) {
         check_cuda(launch_columns_gather_warp(static_cast<int>(w_.ny), nz, zStride, keep_, in, views, tables(), scale,
-                                              twCol_.get(), s),
+                                              twCol_, s),
                    "warp column c2c + retention kernel");
         return;
     }
     if (zStride != nz) throw Error(-3, "padded bin planes need the FP32 warp column kernels");
     check_cuda(launch_columns_gather(p_, static_cast<int>(w_.ny), static_cast<int>(w_.nz), keep_, in, views,
-                                     tables(), scale, colTable_.get(), s),
+                                     tables(), scale, colTable_, s),
                "column c2c + retention kernel");
 }
 
@@ -213,7 +223,7 @@ void HorizontalPlan::inverse_columns_band(DenseBins bins, int slots, int zStride
     if (!bandExact_ || p_ != Precision::f32 || !columns_warp_supported(static_cast<long long>(w_.ny)))
         throw Error(-3, "band column stage needs FP32, an exact retained band and Ny in [32, 512]");
     check_cuda(launch_columns_inverse_band(static_cast<int>(w_.ny), static_cast<int>(w_.nz), zStride, slots, keep_,
-                                           bins, band_.get<int>(), twCol_.get(), colTable_.get(), bandFormInverse_, s),
+                                           bins, band_.get<int>(), twCol_, colTable_, bandFormInverse_, s),
                "band inverse column kernel");
 }
 
@@ -221,7 +231,7 @@ void HorizontalPlan::forward_columns_band(DenseBins bins, int slots, double scal
     if (!bandExact_ || p_ != Precision::f32 || !columns_warp_supported(static_cast<long long>(w_.ny)))
         throw Error(-3, "band column stage needs FP32, an exact retained band and Ny in [32, 512]");
     check_cuda(launch_columns_forward_band(static_cast<int>(w_.ny), static_cast<int>(w_.nz), zStride, slots, keep_,
-                                           bins, band_.get<int>(), scale, twCol_.get(), colTable_.get(), bandFormForward_,
+                                           bins, band_.get<int>(), scale, twCol_, colTable_, bandFormForward_,
                                            s),
                "band forward column kernel");
 }
@@ -229,8 +239,8 @@ void HorizontalPlan::forward_columns_band(DenseBins bins, int slots, double scal
 void HorizontalPlan::inverse_rows(void* real, std::uint64_t planes, cudaStream_t s) const {
     if (planes > maxPlanes_) throw Error(-1, "plane count exceeds the plan's scratch");
     check_cuda(launch_rows_inverse(p_, static_cast<int>(w_.nx), static_cast<int>(w_.ny),
-                                   static_cast<long long>(planes), keep_, scratch(), real, rowInverse_.get(),
-                                   twFull_.get(), s),
+                                   static_cast<long long>(planes), keep_, scratch(), real, rowInverse_,
+                                   twFull_, s),
                "row c2r kernel");
 }
 
@@ -251,10 +261,10 @@ void HorizontalPlan::forward_dense(const void* real, void* wvm, std::uint64_t pl
     if (keep_ != static_cast<int>(w_.nxHalf())) throw Error(-3, "dense transform requested from a pruned plan");
     const DenseBins out{wvm, static_cast<long long>(planes), static_cast<long long>(w_.nxHalf())};
     check_cuda(launch_rows_forward(p_, static_cast<int>(w_.nx), static_cast<int>(w_.ny),
-                                   static_cast<long long>(planes), keep_, real, out, rowForward_.get(), twFull_.get(), s),
+                                   static_cast<long long>(planes), keep_, real, out, rowForward_, twFull_, s),
                "row r2c kernel");
     check_cuda(launch_columns_dense(p_, -1, static_cast<int>(w_.ny), keep_, static_cast<long long>(planes), out, out,
-                                    colTable_.get(), s),
+                                    colTable_, s),
                "column c2c kernel");
 }
 
@@ -263,11 +273,11 @@ void HorizontalPlan::inverse_dense(const void* wvm, void* real, std::uint64_t pl
     if (planes > maxPlanes_) throw Error(-1, "plane count exceeds the plan's scratch");
     const DenseBins in{const_cast<void*>(wvm), static_cast<long long>(planes), static_cast<long long>(w_.nxHalf())};
     check_cuda(launch_columns_dense(p_, +1, static_cast<int>(w_.ny), keep_, static_cast<long long>(planes), in,
-                                    scratch(), colTable_.get(), s),
+                                    scratch(), colTable_, s),
                "column c2c kernel");
     check_cuda(launch_rows_inverse(p_, static_cast<int>(w_.nx), static_cast<int>(w_.ny),
-                                   static_cast<long long>(planes), keep_, scratch(), real, rowInverse_.get(),
-                                   twFull_.get(), s),
+                                   static_cast<long long>(planes), keep_, scratch(), real, rowInverse_,
+                                   twFull_, s),
                "row c2r kernel");
 }
 

@@ -98,7 +98,8 @@ std::uint64_t active_columns(const std::vector<RetainedMode>& modes);
 // grid, a kept kx band and a maximum plane count.
 class HorizontalPlan {
 public:
-    HorizontalPlan(const Workload& w, Precision p, bool pruned, std::uint64_t maxPlanes);
+    // fused: the plan of the fused flux, which has row kernels of its own.
+    HorizontalPlan(const Workload& w, Precision p, bool pruned, std::uint64_t maxPlanes, bool fused = false);
 
     const Workload& workload() const { return w_; }
     Precision precision() const { return p_; }
@@ -152,8 +153,8 @@ public:
     }
     int band_form_inverse() const { return bandFormInverse_; }
     int band_form_forward() const { return bandFormForward_; }
-    const void* twiddlesHalf() const { return twHalf_.get(); }
-    const void* twiddlesFull() const { return twFull_.get(); }
+    const void* twiddlesHalf() const { return twHalf_; }
+    const void* twiddlesFull() const { return twFull_; }
     void embed_dense(const ViewSet& views, void* wvm, std::uint64_t planes, cudaStream_t s) const;
 
     double allocationSeconds = 0.0, planningSeconds = 0.0;
@@ -165,8 +166,12 @@ private:
     int keep_ = 0;
     std::uint64_t maxPlanes_ = 0;
     std::uint64_t modeCount_ = 0;
-    DeviceBuffer twHalf_, twFull_, twCol_;
-    DeviceBuffer rowForward_, rowInverse_, colTable_;  // twHalf / twCol in regs_table_index order
+    // Tables within twiddles_, natural (twHalf, twFull, twCol) or in regs_table_index
+    // order; null where the plan's path does not read them.
+    DeviceBuffer twiddles_;
+    const void *twFull_ = nullptr, *colTable_ = nullptr;
+    const void *twHalf_ = nullptr, *twCol_ = nullptr;            // fused flux
+    const void *rowForward_ = nullptr, *rowInverse_ = nullptr;  // every other path
     DeviceBuffer cellMap_, gatherMap_, colStart_, colKy_, colMode_, modeKx_, modeKy_, modeConj_;
     DeviceBuffer bins_;
     DeviceBuffer band_;

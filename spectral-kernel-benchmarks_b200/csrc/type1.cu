@@ -279,20 +279,19 @@ cudaError_t launch_regs(cx<T>* data, long long seqs, int storage, int first, int
 
 template <typename T>
 cudaError_t launch_t(void* data, long long rows, int nz, int storage, int first, int channels, unsigned mask,
-                     bool norm, const void* twv, const void* tablev, cudaStream_t s) {
+                     bool norm, const void* twv, cudaStream_t s) {
     auto* d = static_cast<cx<T>*>(data);
     const auto* tw = static_cast<const cx<T>*>(twv);
-    const auto* table = static_cast<const cx<T>*>(tablev);
     const long long seqs = rows * channels;
     if (seqs == 0) return cudaSuccess;
     switch (2 * (nz - 1)) {
-        case 8: return launch_regs<T, 8>(d, seqs, storage, first, channels, mask, norm, table, s);
-        case 16: return launch_regs<T, 16>(d, seqs, storage, first, channels, mask, norm, table, s);
-        case 32: return launch_regs<T, 32>(d, seqs, storage, first, channels, mask, norm, table, s);
-        case 64: return launch_regs<T, 64>(d, seqs, storage, first, channels, mask, norm, table, s);
-        case 128: return launch_regs<T, 128>(d, seqs, storage, first, channels, mask, norm, table, s);
-        case 256: return launch_regs<T, 256>(d, seqs, storage, first, channels, mask, norm, table, s);
-        case 512: return launch_regs<T, 512>(d, seqs, storage, first, channels, mask, norm, table, s);
+        case 8: return launch_regs<T, 8>(d, seqs, storage, first, channels, mask, norm, tw, s);
+        case 16: return launch_regs<T, 16>(d, seqs, storage, first, channels, mask, norm, tw, s);
+        case 32: return launch_regs<T, 32>(d, seqs, storage, first, channels, mask, norm, tw, s);
+        case 64: return launch_regs<T, 64>(d, seqs, storage, first, channels, mask, norm, tw, s);
+        case 128: return launch_regs<T, 128>(d, seqs, storage, first, channels, mask, norm, tw, s);
+        case 256: return launch_regs<T, 256>(d, seqs, storage, first, channels, mask, norm, tw, s);
+        case 512: return launch_regs<T, 512>(d, seqs, storage, first, channels, mask, norm, tw, s);
         case 1024: return launch_fft<T, 1024>(d, seqs, storage, first, channels, mask, norm, tw, s);
         default: break;
     }
@@ -317,12 +316,14 @@ bool type1_uses_fft(int nz) {
     return L >= 8 && L <= 1024 && (L & (L - 1)) == 0;
 }
 
+bool type1_uses_regs(std::uint64_t nz) { return nz <= 257 && type1_uses_fft(static_cast<int>(nz)); }
+
 cudaError_t launch_type1(bool f64, void* data, long long rows, int nz, int storageChannels, int first, int channels,
-                         unsigned dstMask, bool normalize, const void* tw, const void* table, cudaStream_t s) {
+                         unsigned dstMask, bool normalize, const void* tw, cudaStream_t s) {
     if (nz < 3 || channels <= 0 || first < 0 || first + channels > storageChannels || channels > 32)
         return cudaErrorInvalidValue;
-    return f64 ? launch_t<double>(data, rows, nz, storageChannels, first, channels, dstMask, normalize, tw, table, s)
-               : launch_t<float>(data, rows, nz, storageChannels, first, channels, dstMask, normalize, tw, table, s);
+    return f64 ? launch_t<double>(data, rows, nz, storageChannels, first, channels, dstMask, normalize, tw, s)
+               : launch_t<float>(data, rows, nz, storageChannels, first, channels, dstMask, normalize, tw, s);
 }
 
 cudaError_t launch_type1_normalize(bool f64, void* data, long long rows, int nz, int storageChannels, int first,

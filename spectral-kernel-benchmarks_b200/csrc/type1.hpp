@@ -15,20 +15,24 @@
 
 #pragma once
 
+#include <cstdint>
+
 #include <cuda_runtime.h>
 
 namespace skb {
 
-// tw: L = 2(nz-1) complex twiddles exp(-2 pi i m / L), m in [0, L), of the
-// handle's precision; table: the same in regs_table_index order of
-// (L, regs_per_thread(L)), read for the power-of-two L up to 512.
+// tw: L = 2(nz-1) complex twiddles exp(-2 pi i m / L) of the handle's precision: m in
+// [0, L), or in regs_table_index order of (L, regs_per_thread(L)) where
+// type1_uses_regs.
 cudaError_t launch_type1(bool f64, void* data, long long rows, int nz, int storageChannels, int first, int channels,
-                         unsigned dstMask, bool normalize, const void* tw, const void* table, cudaStream_t s);
+                         unsigned dstMask, bool normalize, const void* tw, cudaStream_t s);
 // The normalisation alone (the reference's separate adapter pass).
 cudaError_t launch_type1_normalize(bool f64, void* data, long long rows, int nz, int storageChannels, int first,
                                    int channels, unsigned dstMask, cudaStream_t s);
 // True when the transform runs as a 2(nz-1)-point warp FFT of the symmetric
 // extension; other lengths use a direct O(nz^2) sum per column.
 bool type1_uses_fft(int nz);
+// True when that FFT is the register-ended one: the power-of-two L up to 512.
+bool type1_uses_regs(std::uint64_t nz);
 
 }  // namespace skb
