@@ -249,12 +249,16 @@ std::vector<TuneEntry> FluxPipeline::apply_tuned(const void* modalIn, void* moda
                shape + " R=" + std::to_string(g.rows_out()) +
                " S=" + std::to_string(g.inner()) + " groups=" + std::to_string(g.groups()) + dev;
     };
-    const std::vector<int> tileCandidates{4, 8, 16, 32};
-    if (!families_) pick(gemmKey("inverse", *inverseGemm_), tileCandidates, unitTiles(*inverseGemm_), [&] {
+    // Plans on the small-group form have no units: nothing to choose, so the size in
+    // force is the only candidate.
+    auto tileCandidates = [](const VerticalPlan& g) {
+        return g.uses_pipeline() ? std::vector<int>{4, 8, 16, 32} : std::vector<int>{g.unit_tiles()};
+    };
+    if (!families_) pick(gemmKey("inverse", *inverseGemm_), tileCandidates(*inverseGemm_), unitTiles(*inverseGemm_), [&] {
         inverseGemm_->execute({const_cast<void*>(modalIn), nullptr}, {binsIn_.get(), nullptr}, s, M, nullptr,
                               &gemmOut);
     });
-    if (!families_) pick(gemmKey("forward", *forwardGemm_), tileCandidates, unitTiles(*forwardGemm_), [&] {
+    if (!families_) pick(gemmKey("forward", *forwardGemm_), tileCandidates(*forwardGemm_), unitTiles(*forwardGemm_), [&] {
         forwardGemm_->execute({binsOut_.get(), nullptr}, {modalOut, nullptr}, s, M, &gemmIn, nullptr);
     });
     if (cfg_.n == 512) {
