@@ -645,10 +645,11 @@ __global__ void __launch_bounds__(BandRegs<N>::NT, BandRegs<N>::kCtas)
 }
 
 // 512-point band forms with a warp per plane and cp.async staging.
-template <int N, int B>
+template <int B>
 __global__ void __launch_bounds__(32 * B, 4) columns_inverse_band_warp_kernel(int nz, int zStride, DenseBins bins,
                                                                               const int* __restrict__ bandOf,
                                                                               const float2* __restrict__ tw) {
+    constexpr int N = kDirectN;
     constexpr int NT = 32 * B;
     constexpr int XP = plane_region<N>();
     constexpr int ITER = N * B / NT;
@@ -684,11 +685,12 @@ __global__ void __launch_bounds__(32 * B, 4) columns_inverse_band_warp_kernel(in
     }
 }
 
-template <int N, int B>
+template <int B>
 __global__ void __launch_bounds__(32 * B, 4) columns_forward_band_warp_kernel(int nz, int zStride, DenseBins bins,
                                                                               const int* __restrict__ bandOf,
                                                                               float scale,
                                                                               const float2* __restrict__ tw) {
+    constexpr int N = kDirectN;
     constexpr int NT = 32 * B;
     constexpr int XP = plane_region<N>();
     constexpr int ITER = N * B / NT;
@@ -1016,7 +1018,7 @@ cudaError_t inverse_band_512(int nz, int zStride, int slots, int columns, DenseB
         if (err != cudaSuccess) return err;
         kernel<<<grid, 256, kDirectSmem, s>>>(nz, zStride, bins, band, static_cast<const float2*>(tw));
     } else {
-        auto kernel = columns_inverse_band_warp_kernel<kDirectN, B>;
+        auto kernel = columns_inverse_band_warp_kernel<B>;
         const size_t bytes = sizeof(float2) * size_t(B) * plane_region<kDirectN>();
         cudaError_t err = prepare(kernel, bytes);
         if (err != cudaSuccess) return err;
@@ -1046,7 +1048,7 @@ cudaError_t forward_band_512(int nz, int zStride, int slots, int columns, DenseB
         if (err != cudaSuccess) return err;
         kernel<<<grid, 256, kDirectSmem, s>>>(nz, zStride, bins, band, float(scale), static_cast<const float2*>(tw));
     } else {
-        auto kernel = columns_forward_band_warp_kernel<kDirectN, B>;
+        auto kernel = columns_forward_band_warp_kernel<B>;
         const size_t bytes = sizeof(float2) * size_t(B) * plane_region<kDirectN>();
         cudaError_t err = prepare(kernel, bytes);
         if (err != cudaSuccess) return err;

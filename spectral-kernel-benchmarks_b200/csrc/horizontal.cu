@@ -137,7 +137,7 @@ __device__ __forceinline__ void row_forward(cx<T> (&v)[RowShape<T, M>::E], cx<T>
     auto last = [&](int j, V* u) {
 #pragma unroll
         for (int r = 0; r < R; ++r) u[r] = data[S::slot(j + Ns * r, b)];
-        const V* w = tw + regs_table_offset(M, S::E, Ns) + j;
+        const V* w = tw + regs_table_offset(S::E, Ns) + j;
 #pragma unroll
         for (int r = 1; r < R; ++r) u[r] = cmul(u[r], twiddle<-1>(w, Ns * (r - 1)));
         dft_small<-1, R>(u);

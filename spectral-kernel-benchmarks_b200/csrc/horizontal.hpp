@@ -97,10 +97,7 @@ constexpr int regs_table_index(int n, int perThread, int first, int i) {
 }
 // Where the entries of the pass with sub-transform size ns begin (radices
 // perThread, perThread, ... from the first).
-constexpr int regs_table_offset(int n, int perThread, int ns) {
-    (void)n;
-    return ns - perThread;
-}
+constexpr int regs_table_offset(int perThread, int ns) { return ns - perThread; }
 
 // x-direction transforms.  Planes [0, planes) of real volumes laid out
 // [plane][y][x]; bins kept for kx < keep.  twHalf and the column transforms' tw

@@ -115,10 +115,6 @@ __global__ void __launch_bounds__(kWarps * 32) type1_fft_kernel(cx<T>* __restric
     constexpr int M = L / 2;
     constexpr int nz = M + 1;
     constexpr int kSlots = L + L / 16;  // pad16(L - 1) + 1
-    constexpr int kPer = (nz + 31) / 32;  // column values per lane
-    // Up to five values per lane are held for the next column while the
-    // current one is transformed, so its loads overlap the FFT.
-    constexpr bool kPrefetch = kPer <= 5;
     extern __shared__ unsigned char smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long stride = static_cast<long long>(gridDim.x) * kWarps;
@@ -127,37 +123,16 @@ __global__ void __launch_bounds__(kWarps * 32) type1_fft_kernel(cx<T>* __restric
         const long long row = sq / channels;
         return data + (row * storage + first + (sq - row * channels)) * nz;
     };
-    auto load = [&](long long sq, V* v) {
-        const V* col = column(sq);
-#pragma unroll
-        for (int q = 0; q < kPer; ++q) {
-            const int i = lane + 32 * q;
-            v[q] = i < nz ? col[i] : V{T(0), T(0)};
-        }
-    };
-    long long seq = static_cast<long long>(blockIdx.x) * kWarps + warp;
-    V cur[kPrefetch ? kPer : 1];
-    if constexpr (kPrefetch) {
-        if (seq < seqs) load(seq, cur);
-    }
     // Warp-uniform loop; only __syncwarp() is used inside.
-    for (; seq < seqs; seq += stride) {
+    for (long long seq = static_cast<long long>(blockIdx.x) * kWarps + warp; seq < seqs; seq += stride) {
         V* col = column(seq);
         const bool sine = (dstMask >> static_cast<int>(seq % channels)) & 1u;
-        V nxt[kPrefetch ? kPer : 1];
         auto extend = [&](int i, V v) {
             if (sine && (i == 0 || i == M)) v = V{T(0), T(0)};
             x[pad16(i)] = v;
             if (i > 0 && i < M) x[pad16(L - i)] = sine ? V{-v.x, -v.y} : v;
         };
-        if constexpr (kPrefetch) {
-            if (seq + stride < seqs) load(seq + stride, nxt);
-#pragma unroll
-            for (int q = 0; q < kPer; ++q)
-                if (lane + 32 * q < nz) extend(lane + 32 * q, cur[q]);
-        } else {
-            for (int i = lane; i < nz; i += 32) extend(i, col[i]);
-        }
+        for (int i = lane; i < nz; i += 32) extend(i, col[i]);
         __syncwarp();
         warp_fft<T, L, -1>(x, tw, lane);
         for (int k = lane; k < nz; k += 32) {
@@ -166,10 +141,6 @@ __global__ void __launch_bounds__(kWarps * 32) type1_fft_kernel(cx<T>* __restric
             store_result<T>(col, k, y, M, sine, normalize);
         }
         __syncwarp();  // the slot is rewritten by the next column
-        if constexpr (kPrefetch) {
-#pragma unroll
-            for (int q = 0; q < kPer; ++q) cur[q] = nxt[q];
-        }
     }
 }
 

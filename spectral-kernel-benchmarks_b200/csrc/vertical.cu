@@ -21,23 +21,17 @@ constexpr int kTileCols = 32;
 constexpr int kChunk = 32;
 constexpr int kThreads = 256;
 
-template <typename T, bool SPLIT>
-__device__ __forceinline__ cx<T> load_operand(const ComplexOperand& op, long long i) {
-    if (SPLIT) return {reinterpret_cast<const T*>(op.re)[i], reinterpret_cast<const T*>(op.im)[i]};
-    return reinterpret_cast<const cx<T>*>(op.re)[i];
-}
-
-template <typename T, bool SPLIT>
-__device__ __forceinline__ void store_operand(const ComplexOperand& op, long long i, cx<T> v) {
+template <bool SPLIT>
+__device__ __forceinline__ void store_operand(const ComplexOperand& op, long long i, float2 v) {
     if (SPLIT) {
-        reinterpret_cast<T*>(op.re)[i] = v.x;
-        reinterpret_cast<T*>(op.im)[i] = v.y;
+        static_cast<float*>(op.re)[i] = v.x;
+        static_cast<float*>(op.im)[i] = v.y;
     } else {
-        reinterpret_cast<cx<T>*>(op.re)[i] = v;
+        static_cast<float2*>(op.re)[i] = v;
     }
 }
 
-// Asynchronous 4/8/16-byte global->shared copy; src_bytes = 0 writes zeros.
+// Asynchronous 4- or 8-byte global->shared copy; src_bytes = 0 writes zeros.
 template <int BYTES>
 __device__ __forceinline__ void cp_async(void* dst, const void* src, int src_bytes) {
     const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
@@ -50,15 +44,14 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-template <typename T, int KR, bool SPLIT, bool BINS, bool VIRT>
-__global__ void __launch_bounds__(kThreads) grouped_gemm_kernel(int R, int S, const T* __restrict__ At,
+template <int KR, bool SPLIT, bool BINS, bool VIRT>
+__global__ void __launch_bounds__(kThreads) grouped_gemm_kernel(int R, int S, const float* __restrict__ At,
                                                                 GroupTiles tiles, ComplexOperand in,
                                                                 ComplexOperand out, BinBoundary inBins,
                                                                 BinBoundary outBins) {
-    using V = cx<T>;
     constexpr int RP = 32 * KR;
-    constexpr size_t xBytes = sizeof(V) * kTileCols * (kChunk + 1);
-    constexpr size_t aBytes = sizeof(T) * kChunk * RP;
+    constexpr size_t xBytes = sizeof(float2) * kTileCols * (kChunk + 1);
+    constexpr size_t aBytes = sizeof(float) * kChunk * RP;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     // Per tile column: element offsets of the input and output columns (and
     // the output partner), and the conjugation flags.
@@ -113,22 +106,22 @@ __global__ void __launch_bounds__(kThreads) grouped_gemm_kernel(int R, int S, co
         conjOut[c] = cOut ? 1 : 0;
     }
     if (VIRT) __syncwarp();
-    const T* A = At + g * tiles.matrixStride;
+    const float* A = At + g * tiles.matrixStride;
     const int chunks = (S + kChunk - 1) / kChunk;
 
-    auto stageX = [&](int b) { return reinterpret_cast<V(*)[kChunk + 1]>(smem_raw + b * (xBytes + aBytes)); };
-    auto stageA = [&](int b) { return reinterpret_cast<T(*)[RP]>(smem_raw + b * (xBytes + aBytes) + xBytes); };
+    auto stageX = [&](int b) { return reinterpret_cast<float2(*)[kChunk + 1]>(smem_raw + b * (xBytes + aBytes)); };
+    auto stageA = [&](int b) { return reinterpret_cast<float(*)[RP]>(smem_raw + b * (xBytes + aBytes) + xBytes); };
 
     // Issue the copies of chunk c into stage buffer b (zero-filled padding).
     auto issue = [&](int c, int b) {
         const int s0 = c * kChunk;
-        T(*sA)[RP] = stageA(b);
-        V(*sX)[kChunk + 1] = stageX(b);
+        float(*sA)[RP] = stageA(b);
+        float2(*sX)[kChunk + 1] = stageX(b);
         for (int i = threadIdx.x; i < kChunk * RP; i += kThreads) {
             const int s = i / RP, r = i % RP;
             const bool ok = s0 + s < S && r < R;
-            const T* src = ok ? A + (long long)(s0 + s) * R + r : A;
-            cp_async<sizeof(T)>(&sA[s][r], src, ok ? int(sizeof(T)) : 0);
+            const float* src = ok ? A + (long long)(s0 + s) * R + r : A;
+            cp_async<sizeof(float)>(&sA[s][r], src, ok ? int(sizeof(float)) : 0);
         }
         for (int i = threadIdx.x; i < kTileCols * kChunk; i += kThreads) {
             const int c = i / kChunk, s = i % kChunk;
@@ -136,21 +129,21 @@ __global__ void __launch_bounds__(kThreads) grouped_gemm_kernel(int R, int S, co
             const long long idx = ok ? ((VIRT || BINS) ? colIn[c] : (long long)(c0 + c) * S) + s0 + s : 0;
             if (SPLIT) {
                 // Split operands: two scalar copies into the complex slot.
-                T* slot = reinterpret_cast<T*>(&sX[c][s]);
-                cp_async<sizeof(T)>(slot, reinterpret_cast<const T*>(in.re) + idx, ok ? int(sizeof(T)) : 0);
-                cp_async<sizeof(T)>(slot + 1, reinterpret_cast<const T*>(in.im) + idx, ok ? int(sizeof(T)) : 0);
+                float* slot = reinterpret_cast<float*>(&sX[c][s]);
+                cp_async<sizeof(float)>(slot, reinterpret_cast<const float*>(in.re) + idx, ok ? int(sizeof(float)) : 0);
+                cp_async<sizeof(float)>(slot + 1, reinterpret_cast<const float*>(in.im) + idx, ok ? int(sizeof(float)) : 0);
             } else {
-                cp_async<sizeof(V)>(&sX[c][s], reinterpret_cast<const V*>(in.re) + idx, ok ? int(sizeof(V)) : 0);
+                cp_async<sizeof(float2)>(&sX[c][s], reinterpret_cast<const float2*>(in.re) + idx, ok ? int(sizeof(float2)) : 0);
             }
         }
         cp_async_commit();
     };
 
-    V acc[KR][kTileCols / 8];
+    float2 acc[KR][kTileCols / 8];
 #pragma unroll
     for (int k = 0; k < KR; ++k)
 #pragma unroll
-        for (int m = 0; m < kTileCols / 8; ++m) acc[k][m] = {T(0), T(0)};
+        for (int m = 0; m < kTileCols / 8; ++m) acc[k][m] = {0.f, 0.f};
 
     issue(0, 0);
     for (int c = 0; c < chunks; ++c) {
@@ -161,17 +154,17 @@ __global__ void __launch_bounds__(kThreads) grouped_gemm_kernel(int R, int S, co
             cp_async_wait<0>();
         }
         __syncthreads();
-        T(*sA)[RP] = stageA(c & 1);
-        V(*sX)[kChunk + 1] = stageX(c & 1);
+        float(*sA)[RP] = stageA(c & 1);
+        float2(*sX)[kChunk + 1] = stageX(c & 1);
         const int sc = min(kChunk, S - c * kChunk);
 #pragma unroll 4
         for (int s = 0; s < sc; ++s) {
-            T a[KR];
+            float a[KR];
 #pragma unroll
             for (int k = 0; k < KR; ++k) a[k] = sA[s][lane + 32 * k];
 #pragma unroll
             for (int m = 0; m < kTileCols / 8; ++m) {
-                const V x = sX[warp + 8 * m][s];
+                const float2 x = sX[warp + 8 * m][s];
 #pragma unroll
                 for (int k = 0; k < KR; ++k) {
                     acc[k][m].x = fma(a[k], x.x, acc[k][m].x);
@@ -191,56 +184,55 @@ __global__ void __launch_bounds__(kThreads) grouped_gemm_kernel(int R, int S, co
             if (r >= R) continue;
             // The matrices are real, so a conjugated input column gives the
             // conjugate product: both flags are applied here, once.
-            V v = acc[k][m];
+            float2 v = acc[k][m];
             if (!VIRT && !BINS) {
-                store_operand<T, SPLIT>(out, (long long)(c0 + c) * R + r, v);
+                store_operand<SPLIT>(out, (long long)(c0 + c) * R + r, v);
                 continue;
             }
             if (conjIn[c] != conjOut[c]) v.y = -v.y;
-            store_operand<T, SPLIT>(out, colOut[c] + r, v);
-            if (colPartner[c] >= 0) store_operand<T, SPLIT>(out, colPartner[c] + r, V{v.x, -v.y});
+            store_operand<SPLIT>(out, colOut[c] + r, v);
+            if (colPartner[c] >= 0) store_operand<SPLIT>(out, colPartner[c] + r, float2{v.x, -v.y});
         }
     }
 }
 
-template <typename T, int KR>
+template <int KR>
 cudaError_t launch_kr(int R, int S, const void* At, const GroupTiles& tiles, ComplexOperand in, ComplexOperand out,
                       const BinBoundary& inBins, const BinBoundary& outBins, cudaStream_t stream) {
     const bool split = in.im != nullptr;
     if (split != (out.im != nullptr)) return cudaErrorInvalidValue;
-    const size_t bytes = 2 * (sizeof(cx<T>) * kTileCols * (kChunk + 1) + sizeof(T) * kChunk * 32 * KR);
+    const size_t bytes = 2 * (sizeof(float2) * kTileCols * (kChunk + 1) + sizeof(float) * kChunk * 32 * KR);
     const bool bins = inBins.cell != nullptr || outBins.cell != nullptr;
-    using K = void (*)(int, int, const T*, GroupTiles, ComplexOperand, ComplexOperand, BinBoundary, BinBoundary);
+    using K = void (*)(int, int, const float*, GroupTiles, ComplexOperand, ComplexOperand, BinBoundary, BinBoundary);
     // [split][bins][virtual]
     const K kernels[2][2][2] = {
-        {{grouped_gemm_kernel<T, KR, false, false, false>, grouped_gemm_kernel<T, KR, false, false, true>},
-         {grouped_gemm_kernel<T, KR, false, true, false>, grouped_gemm_kernel<T, KR, false, true, true>}},
-        {{grouped_gemm_kernel<T, KR, true, false, false>, grouped_gemm_kernel<T, KR, true, false, true>},
-         {grouped_gemm_kernel<T, KR, true, true, false>, grouped_gemm_kernel<T, KR, true, true, true>}}};
+        {{grouped_gemm_kernel<KR, false, false, false>, grouped_gemm_kernel<KR, false, false, true>},
+         {grouped_gemm_kernel<KR, false, true, false>, grouped_gemm_kernel<KR, false, true, true>}},
+        {{grouped_gemm_kernel<KR, true, false, false>, grouped_gemm_kernel<KR, true, false, true>},
+         {grouped_gemm_kernel<KR, true, true, false>, grouped_gemm_kernel<KR, true, true, true>}}};
     const K kernel = kernels[split][bins][tiles.virtualColumns];
     if (bytes > 48 * 1024) {
         const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
         if (err != cudaSuccess) return err;
     }
-    kernel<<<tiles.tiles, kThreads, bytes, stream>>>(R, S, static_cast<const T*>(At), tiles, in, out, inBins,
+    kernel<<<tiles.tiles, kThreads, bytes, stream>>>(R, S, static_cast<const float*>(At), tiles, in, out, inBins,
                                                      outBins);
     return cudaGetLastError();
 }
 
-template <typename T>
-cudaError_t launch_t(int R, int S, const void* At, const GroupTiles& tiles, ComplexOperand in, ComplexOperand out,
+cudaError_t launch_f32(int R, int S, const void* At, const GroupTiles& tiles, ComplexOperand in, ComplexOperand out,
                      const BinBoundary& ib, const BinBoundary& ob, cudaStream_t stream) {
     const int kr = (R + 31) / 32;
     switch (kr) {
-        case 1: return launch_kr<T, 1>(R, S, At, tiles, in, out, ib, ob, stream);
-        case 2: return launch_kr<T, 2>(R, S, At, tiles, in, out, ib, ob, stream);
-        case 3: return launch_kr<T, 3>(R, S, At, tiles, in, out, ib, ob, stream);
-        case 4: return launch_kr<T, 4>(R, S, At, tiles, in, out, ib, ob, stream);
-        case 5: return launch_kr<T, 5>(R, S, At, tiles, in, out, ib, ob, stream);
-        case 6: return launch_kr<T, 6>(R, S, At, tiles, in, out, ib, ob, stream);
+        case 1: return launch_kr<1>(R, S, At, tiles, in, out, ib, ob, stream);
+        case 2: return launch_kr<2>(R, S, At, tiles, in, out, ib, ob, stream);
+        case 3: return launch_kr<3>(R, S, At, tiles, in, out, ib, ob, stream);
+        case 4: return launch_kr<4>(R, S, At, tiles, in, out, ib, ob, stream);
+        case 5: return launch_kr<5>(R, S, At, tiles, in, out, ib, ob, stream);
+        case 6: return launch_kr<6>(R, S, At, tiles, in, out, ib, ob, stream);
         case 7:
         case 8:
-        case 9: return launch_kr<T, 9>(R, S, At, tiles, in, out, ib, ob, stream);
+        case 9: return launch_kr<9>(R, S, At, tiles, in, out, ib, ob, stream);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -258,7 +250,7 @@ cudaError_t launch_grouped_gemm(GemmPrecision p, int R, int S, const void* matri
     switch (p) {
         case GemmPrecision::f64:
             return launch_grouped_gemm_f64(R, S, static_cast<const double*>(matrices), tiles, in, out, ib, ob, stream);
-        case GemmPrecision::f32: return launch_t<float>(R, S, matrices, tiles, in, out, ib, ob, stream);
+        case GemmPrecision::f32: return launch_f32(R, S, matrices, tiles, in, out, ib, ob, stream);
         default: return cudaErrorNotSupported;
     }
 }
