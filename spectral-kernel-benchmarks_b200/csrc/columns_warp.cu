@@ -597,7 +597,9 @@ __global__ void __launch_bounds__(256, 2) columns_band_persist_kernel(int nz, in
 // HBM (54 %).  256 points, 48 slots of 65 planes (835 MB): inverse 320 -> 205 us,
 // forward (12 slots) 81 -> 51 us; 128 points, 12 slots of 33: 19 -> 12 us.  At 512
 // points (15 slots of 129) 559 us against 532 of the pipelined form, forward (4
-// slots) 138 us against 146 of the next best: a tuner candidate.
+// slots) 138 us against 146 of the next best: a tuner candidate, and the forward form
+// of untuned handles.  The cap of 64 registers (1,024 resident threads) costs 16 to 40
+// bytes of spills from 128 points on.
 template <int N>
 struct BandRegs {
     static constexpr int B = 16;

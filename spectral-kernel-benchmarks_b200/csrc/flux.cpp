@@ -180,12 +180,13 @@ FluxPipeline::FluxPipeline(const FluxConfig& cfg) : cfg_(cfg) {
     if (fused_ && dense_ && cfg.n == 512) {
         // Forms of an untuned handle, the autotuner's usual picks.  Rows: two
         // planes per warp, three CTAs per SM, TMA stages (one member, Nz 129:
-        // 997 us warp per plane -> 765).  Columns: the pipelined form walking
-        // 16 columns from 128 chunks of 16 planes on, where its one CTA per SM
-        // has several waves (15 slots of 129, one member: direct 697 us, 16
-        // planes 570, pipelined 532; 12 slots of 33: 150, 144, 165); forward
-        // from there on either 16-plane form, register-ended below (4 slots of
-        // 129: 138 us against 146 and 156).
+        // 997 us warp per plane -> 765).  Inverse columns: the pipelined form
+        // walking 16 columns from 127 full chunks of 16 planes on, where its one
+        // CTA per SM has several waves, the plain 16-plane form below.  The line is
+        // the smaller of the two sizes timed: 15 slots of 129, one member (127.5
+        // chunks): direct 697 us, 16 planes 570, pipelined 532; 12 slots of 33 (30
+        // chunks): 150, 144, 165.  Forward columns: register-ended at every size (4
+        // slots of 129: 138 us, pipelined 146, 16 planes 156).
         rowsPairs_ = 2;
         rowsTma_ = 1;
         const std::uint64_t inChunks = cfg.members * fieldsIn_ * zStride_ / 16;

@@ -20,7 +20,9 @@ constexpr int phase_lanes() {
 
 // Resident CTAs per SM that a kernel is compiled for: what
 // shared memory, the registers it needs (per thread, by elements held) and the
-// thread limit allow.
+// thread limit allow.  At these counts ptxas
+// spills 32 bytes in the 256-point FP64 inverse rows, 8 and 24 in the 128-point FP32
+// columns of the pruned transforms and 4 or 8 in five other FP64 kernels.
 template <typename T>
 constexpr int resident_ctas(int threads, size_t bytes, int elements) {
     const int regs = sizeof(T) == 8 ? (elements > 8 ? 96 : 64) : (elements > 8 ? 56 : 40);
@@ -364,12 +366,14 @@ __global__ void __launch_bounds__(RowShape<T, M>::NT, RowShape<T, M>::kCtas)
 //   bins(m, z) <- r2c(-scale (u q_x + v q_y + w q_z)),  q_f = c2r(bins(3 m + f, z)).
 // Neither the derivatives' real rows nor the product's are stored: 8 of the 11 real
 // volumes that inverse rows, pointwise product and forward rows moved per target.
-// Bound: latency, at two CTAs of 128 threads per SM (FP64, 255 registers: the sum, a
-// slot's row and the velocity row in flight), 3.6 TB/s.  Row stages of a flux, before
+// Bound: latency, at two CTAs of 128 threads per SM (FP64, 255 registers and, at 512
+// points, 100 bytes of spills: the sum, a slot's row and the velocity row in flight; FP32
+// at 512 points 128 registers and 56 bytes), 3.6 TB/s.  Row stages of a flux, before
 // and now: FP64 512^2, Nz 129, 4 targets 2869 -> 2005 us, 256^2, Nz 65, 3 targets of 2
 // members 597 -> 390; FP32 512^2, Nz 65 842 -> 686, 256^2 337 -> 225; FP64 1024^2, Nz
 // 17 1324 -> 1235, FP32 836 -> 877 (1141 with every pass of the rows in shared
-// memory).  512^2 without the L2 prefetches 2400, with 168 registers for a third CTA
+// memory).  The row bodies shared with this kernel made the plain row kernels up to
+// 2 % slower (FP32 256^2 pruned round trip 60.4 -> 61.7 us, FP64 256^2 FFT 166.5 -> 168).  512^2 without the L2 prefetches 2400, with 168 registers for a third CTA
 // (spills) 2037-2051.
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 

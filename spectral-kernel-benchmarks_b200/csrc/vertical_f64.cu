@@ -19,9 +19,10 @@
 // (FMA instructions 34.1) and a warp's 18 of them per step of 4 take 11 shared
 // loads.  The FMA form before it padded rows to 32 and was held at 39-46 % of
 // the FP64 pipe by shared loads and 8-byte copies.  Both directions at 256^2,
-// Nz 65, 3 fields (2,045 groups of 17 columns): 156 -> 74 us; 512^2, Nz 129:
+// Nz 65, 3 fields (2,045 groups of 17 columns): 156 -> 64 us; 512^2, Nz 129:
 // 15-field inverse 2.14 -> 1.43 ms, 4-field forward 0.82 -> 0.42 ms.  Persistent
-// CTAs with the copies running across tiles: 77 us, and 1 % slower at 512^2.
+// CTAs with the copies running across tiles: 77 us (against 74 before a warp copied
+// whole columns), and 1 % slower at 512^2.
 
 #include "launch.cuh"
 #include "vertical_device.cuh"
