@@ -20,7 +20,7 @@
 // loads.  The FMA form before it padded rows to 32 and was held at 39-46 % of
 // the FP64 pipe by shared loads and 8-byte copies.  Both directions at 256^2,
 // Nz 65, 3 fields (2,045 groups of 17 columns): 156 -> 64 us; 512^2, Nz 129:
-// 15-field inverse 2.14 -> 1.43 ms, 4-field forward 0.82 -> 0.42 ms.  Persistent
+// 15-field inverse 2.14 -> 1.27 ms, 4-field forward 0.82 -> 0.37 ms.  Persistent
 // CTAs with the copies running across tiles: 77 us (against 74 before a warp copied
 // whole columns), and 1 % slower at 512^2.
 
